@@ -174,20 +174,15 @@ __device__ __forceinline__ double adj_pair(const TileGate& g, int mode, double* 
                                            uint32_t nw) {
   const Enumerator<NPOS, TileGate> E(g);
   const uint32_t tbit = g.tbit;
-  const Coef cf = g.c;
+  const PairGate<KIND> op(g.c);
   double acc = 0.0;
   for (uint32_t m = threadIdx.x; m < nw; m += blockDim.x) {
     const uint32_t s0 = E(m), s1 = s0 | tbit;
     double a = pr[s0], b = pi[s0], c = pr[s1], d = pi[s1];
     double p = lr[s0], q = li[s0], r = lr[s1], s = li[s1];
     if (mode >= 0) acc = dadd(acc, adj_pair_term(mode, a, b, c, d, p, q, r, s));
-    if constexpr (KIND >= FK_LAZY_H) {
-      fast_pair<KIND>(cf, a, b, c, d);
-      fast_pair<KIND>(cf, p, q, r, s);
-    } else {
-      gate_pair<KIND>(cf, a, b, c, d);
-      gate_pair<KIND>(cf, p, q, r, s);
-    }
+    op(a, b, c, d);
+    op(p, q, r, s);
     pr[s0] = a; pi[s0] = b; pr[s1] = c; pi[s1] = d;
     lr[s0] = p; li[s0] = q; lr[s1] = r; li[s1] = s;
   }
@@ -203,7 +198,7 @@ __device__ __forceinline__ double adj_diag(const TileGate& g, int mode, int glob
                                            double* lr, double* li, uint32_t nw) {
   const Enumerator<NPOS, TileGate> E(g);
   const uint32_t tbit = g.tbit;
-  const Coef cf = g.c;
+  const DiagGate<KIND> op(g.c);
   double acc = 0.0;
   for (uint32_t m = threadIdx.x; m < nw; m += blockDim.x) {
     const uint32_t e = E(m);
@@ -213,8 +208,8 @@ __device__ __forceinline__ double adj_diag(const TileGate& g, int mode, int glob
       const double v = dfma(p, b, dmul(dneg(q), a));  // Im(conj(lam) psi)
       acc = (mode == GM_Z && one) ? dsub(acc, v) : dadd(acc, v);
     }
-    gate_diag<KIND>(cf, one, a, b);
-    gate_diag<KIND>(cf, one, p, q);
+    op(one, a, b);
+    op(one, p, q);
     pr[e] = a; pi[e] = b; lr[e] = p; li[e] = q;
   }
   return acc;

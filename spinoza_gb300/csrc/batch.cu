@@ -218,7 +218,7 @@ __device__ __forceinline__ double b_bwd_pair(const BGate& g, double* pr, double*
                                              uint32_t nw) {
   const Enumerator<NPOS, BGate> E(g);
   const uint32_t tbit = g.tbit;
-  const Coef cf = g.c;
+  const PairGate<KIND> op(g.c);
   const int grad = g.grad;
   double acc = 0.0;
   for (uint32_t m = threadIdx.x; m < nw; m += blockDim.x) {
@@ -235,8 +235,8 @@ __device__ __forceinline__ double b_bwd_pair(const BGate& g, double* pr, double*
       }
       acc = dadd(acc, v);
     }
-    gate_pair<KIND>(cf, a, b, c, d);
-    gate_pair<KIND>(cf, p, q, r, s);
+    op(a, b, c, d);
+    op(p, q, r, s);
     pr[s0] = a; pi[s0] = b; pr[s1] = c; pi[s1] = d;
     lr[s0] = p; li[s0] = q; lr[s1] = r; li[s1] = s;
   }
@@ -248,7 +248,7 @@ __device__ __forceinline__ double b_bwd_diag(const BGate& g, int gone, double* p
                                              uint32_t nw) {
   const Enumerator<NPOS, BGate> E(g);
   const uint32_t tbit = g.tbit;
-  const Coef cf = g.c;
+  const DiagGate<KIND> op(g.c);
   const int grad = g.grad;
   double acc = 0.0;
   for (uint32_t m = threadIdx.x; m < nw; m += blockDim.x) {
@@ -259,8 +259,8 @@ __device__ __forceinline__ double b_bwd_diag(const BGate& g, int gone, double* p
       const double v = dfma(p, b, dmul(dneg(q), a));  // Im(conj(lam) psi)
       acc = (grad == BG_Z && one) ? dsub(acc, v) : dadd(acc, v);
     }
-    gate_diag<KIND>(cf, one, a, b);
-    gate_diag<KIND>(cf, one, p, q);
+    op(one, a, b);
+    op(one, p, q);
     pr[e] = a; pi[e] = b; lr[e] = p; li[e] = q;
   }
   return acc;

@@ -168,17 +168,10 @@ struct PairArgs {
   uint8_t pos[kMaxQubits + 2];
 };
 
-// Exact gates use the reference's arithmetic; the lazy kinds (FK_LAZY_*, the
-// gate divided by a scalar) use the 4-instruction forms.
-template <int KIND>
-__device__ __forceinline__ void pair_op(const Coef& c, double& a, double& b, double& x, double& d) {
-  if constexpr (KIND >= FK_LAZY_H) fast_pair<KIND>(c, a, b, x, d);
-  else gate_pair<KIND>(c, a, b, x, d);
-}
-
 // Two consecutive pairs per thread; requires every special position >= 1.
 template <int KIND>
 __global__ void __launch_bounds__(kThreads) pair_kernel_v2(PairArgs A) {
+  const PairGate<KIND> op(A.c);
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < A.nwork; w += stride) {
     const uint64_t s0 = deposit(2 * w, A.pos, A.npos) | A.ones;
@@ -187,8 +180,8 @@ __global__ void __launch_bounds__(kThreads) pair_kernel_v2(PairArgs A) {
     double2 i0 = *reinterpret_cast<const double2*>(A.im + s0);
     double2 r1 = *reinterpret_cast<const double2*>(A.re + s1);
     double2 i1 = *reinterpret_cast<const double2*>(A.im + s1);
-    pair_op<KIND>(A.c, r0.x, i0.x, r1.x, i1.x);
-    pair_op<KIND>(A.c, r0.y, i0.y, r1.y, i1.y);
+    op(r0.x, i0.x, r1.x, i1.x);
+    op(r0.y, i0.y, r1.y, i1.y);
     *reinterpret_cast<double2*>(A.re + s0) = r0;
     *reinterpret_cast<double2*>(A.im + s0) = i0;
     *reinterpret_cast<double2*>(A.re + s1) = r1;
@@ -199,12 +192,13 @@ __global__ void __launch_bounds__(kThreads) pair_kernel_v2(PairArgs A) {
 // Target 0 (no control on bit 0): the pair (s0, s0 + 1) is one double2.
 template <int KIND>
 __global__ void __launch_bounds__(kThreads) pair_kernel_t0(PairArgs A) {
+  const PairGate<KIND> op(A.c);
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < A.nwork; w += stride) {
     const uint64_t s0 = deposit(w, A.pos, A.npos) | A.ones;
     double2 r = *reinterpret_cast<const double2*>(A.re + s0);
     double2 i = *reinterpret_cast<const double2*>(A.im + s0);
-    pair_op<KIND>(A.c, r.x, i.x, r.y, i.y);
+    op(r.x, i.x, r.y, i.y);
     *reinterpret_cast<double2*>(A.re + s0) = r;
     *reinterpret_cast<double2*>(A.im + s0) = i;
   }
@@ -213,12 +207,13 @@ __global__ void __launch_bounds__(kThreads) pair_kernel_t0(PairArgs A) {
 // Scalar form (a control on bit 0).
 template <int KIND>
 __global__ void __launch_bounds__(kThreads) pair_kernel_s(PairArgs A) {
+  const PairGate<KIND> op(A.c);
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < A.nwork; w += stride) {
     const uint64_t s0 = deposit(w, A.pos, A.npos) | A.ones;
     const uint64_t s1 = s0 | A.tbit;
     double a = A.re[s0], b = A.im[s0], c = A.re[s1], d = A.im[s1];
-    pair_op<KIND>(A.c, a, b, c, d);
+    op(a, b, c, d);
     A.re[s0] = a;
     A.im[s0] = b;
     A.re[s1] = c;
@@ -230,13 +225,14 @@ __global__ void __launch_bounds__(kThreads) pair_kernel_s(PairArgs A) {
 // own target bit picks the diagonal entry.
 template <int KIND>
 __global__ void __launch_bounds__(kThreads) diag_kernel_v2(PairArgs A) {
+  const DiagGate<KIND> op(A.c);
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < A.nwork; w += stride) {
     const uint64_t e = deposit(2 * w, A.pos, A.npos) | A.ones;
     double2 r = *reinterpret_cast<const double2*>(A.re + e);
     double2 i = *reinterpret_cast<const double2*>(A.im + e);
-    gate_diag<KIND>(A.c, (e & A.tbit) != 0, r.x, i.x);
-    gate_diag<KIND>(A.c, ((e + 1) & A.tbit) != 0, r.y, i.y);
+    op((e & A.tbit) != 0, r.x, i.x);
+    op(((e + 1) & A.tbit) != 0, r.y, i.y);
     *reinterpret_cast<double2*>(A.re + e) = r;
     *reinterpret_cast<double2*>(A.im + e) = i;
   }
@@ -244,11 +240,12 @@ __global__ void __launch_bounds__(kThreads) diag_kernel_v2(PairArgs A) {
 
 template <int KIND>
 __global__ void __launch_bounds__(kThreads) diag_kernel_s(PairArgs A) {
+  const DiagGate<KIND> op(A.c);
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < A.nwork; w += stride) {
     const uint64_t e = deposit(w, A.pos, A.npos) | A.ones;
     double r = A.re[e], i = A.im[e];
-    gate_diag<KIND>(A.c, (e & A.tbit) != 0, r, i);
+    op((e & A.tbit) != 0, r, i);
     A.re[e] = r;
     A.im[e] = i;
   }

@@ -94,7 +94,7 @@ template <int KIND, int NPOS, class G, class SW = NoSwizzle>
 __device__ __forceinline__ void tile_pair(const G& g, double* sre, double* sim, uint32_t npairs) {
   const Enumerator<NPOS, G> E(g);
   const uint32_t tbit = g.tbit;
-  const Coef c = g.c;
+  const PairGate<KIND> op(g.c);
   if constexpr (kTileBatch > 1) {
     const uint32_t step = blockDim.x;
     for (uint32_t m0 = threadIdx.x; m0 < npairs; m0 += kTileBatch * step) {
@@ -109,10 +109,7 @@ __device__ __forceinline__ void tile_pair(const G& g, double* sre, double* sim, 
         a[u] = sre[s0[u]]; b[u] = sim[s0[u]]; x[u] = sre[s1[u]]; d[u] = sim[s1[u]];
       }
 #pragma unroll
-      for (int u = 0; u < kTileBatch; ++u) {
-        if constexpr (KIND >= FK_LAZY_H) fast_pair<KIND>(c, a[u], b[u], x[u], d[u]);
-        else gate_pair<KIND>(c, a[u], b[u], x[u], d[u]);
-      }
+      for (int u = 0; u < kTileBatch; ++u) op(a[u], b[u], x[u], d[u]);
 #pragma unroll
       for (int u = 0; u < kTileBatch; ++u) {
         if (m0 + u * step < npairs) {
@@ -126,8 +123,7 @@ __device__ __forceinline__ void tile_pair(const G& g, double* sre, double* sim, 
       const uint32_t e0 = E(m);
       const uint32_t s0 = SW::at(e0), s1 = SW::at(e0 | tbit);
       double a = sre[s0], b = sim[s0], x = sre[s1], d = sim[s1];
-      if constexpr (KIND >= FK_LAZY_H) fast_pair<KIND>(c, a, b, x, d);
-      else gate_pair<KIND>(c, a, b, x, d);
+      op(a, b, x, d);
       sre[s0] = a; sim[s0] = b; sre[s1] = x; sim[s1] = d;
     }
   }
@@ -144,13 +140,13 @@ template <int KIND, int NPOS, class G, class SW = NoSwizzle>
 __device__ __forceinline__ void tile_diag(const G& g, double* sre, double* sim, uint32_t nelem, int global_one) {
   const Enumerator<NPOS, G> E(g);
   const uint32_t tbit = g.tbit;
-  const Coef c = g.c;
+  const DiagGate<KIND> op(g.c);
   for (uint32_t m = threadIdx.x; m < nelem; m += blockDim.x) {
     const uint32_t e0 = E(m);
     const bool one = global_one >= 0 ? global_one != 0 : (e0 & tbit) != 0;
     const uint32_t e = SW::at(e0);
     double r = sre[e], i = sim[e];
-    gate_diag<KIND>(c, one, r, i);
+    op(one, r, i);
     sre[e] = r; sim[e] = i;
   }
 }
