@@ -413,7 +413,9 @@ typedef struct spz_batch_config {
   int32_t threads;        /* threads per CTA, multiple of 32 in 64..1024 (0 = 64) */
   int32_t wide_qubits;    /* instances of at least this many qubits (and more than
                              tile_qubits) are split into work items across CTAs, each
-                             with its own psi and lam in HBM; 0 = 18, > 30 = never.
+                             with its own psi and lam in HBM; 0 = 18 and up, and smaller
+                             ones (10 and up) that one CTA alone would hold the launch
+                             up with; > 30 = never.
                              Those whose workspace exceeds 60% of free memory, and all
                              of them under SPZ_EXEC_FAST, run one at a time across
                              the GPU instead (fused executor + fused adjoint sweep) */
@@ -422,7 +424,8 @@ typedef struct spz_batch_config {
                              across the GPU; SPZ_BATCH_WIDE_APART: the wide instances
                              run one at a time across the GPU in the exact mode too
                              (no per-instance workspace held for the whole run)      */
-  int32_t tiles_per_item; /* tiles per work item of a wide instance (0 = 64)       */
+  int32_t tiles_per_item; /* tiles per work item of a wide instance (0 = chosen to
+                             fill the GPU, at most 64)                              */
 } spz_batch_config;
 
 #define SPZ_BATCH_WIDE_APART 16

@@ -57,13 +57,25 @@ constexpr uint64_t kWorkspaceBudget = 128ull << 30;  // HBM for streamed instanc
 // does better.  4096 instances of 10-22 qubits measured 32.5 s with
 // the persistent kernel alone and 26.1-26.7 s with the threshold at 17-20.
 constexpr int kDefaultWideQubits = 18;
+// A smaller instance is spread over CTAs too when running it whole would take
+// one CTA more than this share of the launch (its cost times the CTA slots
+// over the batch's cost): with few instances the largest whole one is the
+// launch's serial tail.  Measured, 256 instances of 8-18 qubits: 848 ms with
+// only 18 qubits and up spread, 66 ms with this rule; 1024 of 10-17: 1269
+// and 198 ms; 64 of 4-11: 4.6 and 1.6 ms; in a batch of thousands
+// the rule changes little (the tail is short against the whole).  Instances
+// under kMinSpreadQubits stay whole: a pass over them is too short to share.
+constexpr double kWholeShare = 0.25;
+constexpr uint32_t kMinSpreadQubits = 10;
 constexpr int kWideStreams = 4;         // at most this many wide instances in flight (whole-GPU path)
 constexpr int kDefaultWideStreams = 3;  // SPZ_BATCH_WIDE_STREAMS in the environment overrides it (1..4)
 // Tiles per work item of a wide instance (2^9-amplitude tiles: 64 tiles of a
-// 22-qubit pass make 128 items).  The 4096-instance batch of 10-22 qubits
-// measured 25.65 s with 64, 25.71 s
-// with 16, 25.83 s with 4.
-constexpr int kDefaultTilesPerItem = 64;
+// 22-qubit pass make 128 items), at most: the 4096-instance batch of 10-22
+// qubits measured 25.65 s with 64, 25.71 s with 16, 25.83 s with 4.  Fewer
+// when one pass of every wide instance would make less than kItemsPerSlot
+// items per CTA slot, so that small batches still fill the GPU.
+constexpr int kMaxTilesPerItem = 64;
+constexpr int kItemsPerSlot = 4;
 // Polls (about 0.3 us each) before a dependency wait gives up: far longer
 // than any item takes, short enough that a lost dependency ends the launch.
 constexpr unsigned long long kDefaultWaitPolls = 1ull << 24;
@@ -717,6 +729,7 @@ struct BatchImpl {
   // 128, 28.2 s with 2^11 x 128, 26.9 s with 2^9 x 128 and with 2^8 x 64.
   int kmax = 9, threads = 64;
   int wide_qubits = kDefaultWideQubits;
+  bool wide_auto = true;              // no threshold given: smaller instances by cost too (kWholeShare)
   uint32_t wide_flags = 0;            // SPZ_EXEC_FAST: wide instances use the fast adjoint
   uint32_t nnarrow = 0;               // instances in the persistent kernel
   std::vector<WideInst> wide;         // the others, largest first
@@ -734,7 +747,7 @@ struct BatchImpl {
   size_t smem = 0;
   cudaStream_t stream = nullptr;
   // wide instances inside the persistent kernel (work items)
-  int tiles_per_item = kDefaultTilesPerItem;
+  int tiles_per_item = 0;             // 0: chosen in build_batch
   uint32_t nitems = 0, nwide_items = 0, nwide_in_kernel = 0, nsums = 0;
   uint64_t npartials = 0, wide_ws_doubles = 0;
   unsigned long long wait_limit = kDefaultWaitPolls;
@@ -817,6 +830,21 @@ int build_batch(spz_batch_t b, const spz_batch_instance* inst, size_t ninst, con
   SPZ_CUDA(cudaMemGetInfo(&free_b, &total_b));
   const uint64_t wide_budget = (uint64_t)(kWideWorkspaceShare * (double)free_b);
   uint64_t wide_ws = 0;
+  // launch shape: persistent CTAs, as many per SM as shared memory allows
+  const uint32_t TMAX = 1u << b->kmax;
+  b->smem = (4 * TMAX + ((2 * TMAX) >> kBatchLowBits) + (size_t)(b->threads / 32) * (1 + kMaxPassParams)) *
+            sizeof(double);
+  const void* kfn = batch_kernel_fn(b->threads);
+  SPZ_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->smem));
+  int per_sm = 0, sms = 0;
+  SPZ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, b->threads, b->smem));
+  if (per_sm < 1) return fail(SPZ_ERR_UNSUPPORTED, "batch kernel does not fit on an SM with this configuration");
+  SPZ_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device));
+  const double slots_of_gpu = (double)sms * per_sm;
+  double total_cost = 0.0;
+  for (size_t ii = 0; ii < ninst; ++ii)
+    if (inst[ii].n <= 30) total_cost += (double)(inst[ii].nops + 8) * (double)(1ull << inst[ii].n);
+  const bool by_cost = b->wide_auto && !(b->wide_flags & (SPZ_EXEC_FAST | SPZ_BATCH_WIDE_APART));
   for (size_t ii = 0; ii < ninst; ++ii) {
     const spz_batch_instance& in = inst[ii];
     const uint32_t n = in.n;
@@ -824,10 +852,14 @@ int build_batch(spz_batch_t b, const spz_batch_instance* inst, size_t ninst, con
     // Wide instances run as work items inside the persistent kernel, with
     // their own psi and lam in HBM, when the workspace fits; the fast adjoint
     // (SPZ_EXEC_FAST) and anything beyond the budget take the whole-GPU path.
-    const bool wide = (int)n >= b->wide_qubits && (int)n > b->kmax;
+    const bool costly = by_cost && n >= kMinSpreadQubits &&
+                        (double)(in.nops + 8) * (double)(1ull << n) * slots_of_gpu > kWholeShare * total_cost;
+    const bool large = (int)n >= b->wide_qubits;
+    bool wide = (large || costly) && (int)n > b->kmax;
     const uint64_t ws_need = 4ull * (1ull << n);
     const bool in_kernel = wide && !(b->wide_flags & (SPZ_EXEC_FAST | SPZ_BATCH_WIDE_APART)) &&
                            (wide_ws + ws_need) * 8 <= wide_budget;
+    wide = wide && (in_kernel || large);  // beyond the budget a smaller instance runs whole
     if (wide && in_kernel) {
       wide_index[ii] = (int32_t)wide_in.size();
       wide_in.push_back((uint32_t)ii);
@@ -1075,7 +1107,12 @@ int build_batch(spz_batch_t b, const spz_batch_instance* inst, size_t ninst, con
   std::vector<std::vector<uint64_t>> pass_slot(ninst);
   uint64_t nslots = 0;
   uint32_t max_pass = 0;
-  const uint64_t tpi = (uint64_t)std::max(1, b->tiles_per_item);
+  if (b->tiles_per_item == 0) {
+    double wide_tiles = 0.0;
+    for (uint32_t ii : wide_in) wide_tiles += (double)(1ull << (inst[ii].n - b->kmax));
+    b->tiles_per_item = (int)std::min<double>(kMaxTilesPerItem, std::max(1.0, wide_tiles / (kItemsPerSlot * slots_of_gpu)));
+  }
+  const uint64_t tpi = (uint64_t)b->tiles_per_item;
   uint64_t ws_off = 0;
   for (uint32_t ii : worder) {
     BInst& I = vinst[ii];
@@ -1158,17 +1195,6 @@ int build_batch(spz_batch_t b, const spz_batch_instance* inst, size_t ninst, con
   SPZ_CUDA(host_alloc(&b->h_theta, std::max<uint64_t>(1, ptotal) * sizeof(double)));
   SPZ_CUDA(host_alloc(&b->h_grad, std::max<uint64_t>(1, ptotal) * sizeof(double)));
   SPZ_CUDA(host_alloc(&b->h_energy, std::max<size_t>(1, ninst) * sizeof(double)));
-  // launch shape: persistent CTAs, as many per SM as shared memory allows
-  const uint32_t TMAX = 1u << b->kmax;
-  b->smem = (4 * TMAX + ((2 * TMAX) >> kBatchLowBits) + (size_t)(b->threads / 32) * (1 + kMaxPassParams)) *
-            sizeof(double);
-  const void* kfn = batch_kernel_fn(b->threads);
-  SPZ_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->smem));
-  int per_sm = 0;
-  SPZ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, b->threads, b->smem));
-  if (per_sm < 1) return fail(SPZ_ERR_UNSUPPORTED, "batch kernel does not fit on an SM with this configuration");
-  int sms = 0;
-  SPZ_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device));
   b->grid = std::max(1, std::min<int>(sms * per_sm, (int)b->nitems));
   if (ws_qubits) {
     // Each CTA owns psi and lam of the largest streamed instance; keep the
@@ -1244,9 +1270,16 @@ int spz_batch_create(const spz_batch_instance* instances, size_t ninstances, con
   if (config) {
     if (config->tile_qubits) b->kmax = config->tile_qubits;
     if (config->threads) b->threads = config->threads;
-    if (config->wide_qubits) b->wide_qubits = config->wide_qubits;
+    if (config->wide_qubits) {
+      b->wide_qubits = config->wide_qubits;
+      b->wide_auto = false;
+    }
     b->wide_flags = (uint32_t)config->flags & (SPZ_EXEC_FAST | SPZ_BATCH_WIDE_APART);
-    if (config->tiles_per_item) b->tiles_per_item = config->tiles_per_item;
+    if (config->tiles_per_item < 0) {
+      delete b;
+      return fail(SPZ_ERR_INVALID_ARGUMENT, "batch config: tiles_per_item must be >= 1");
+    }
+    b->tiles_per_item = config->tiles_per_item;
   }
   {
     const char* v = std::getenv("SPZ_BATCH_WIDE_STREAMS");
@@ -1258,10 +1291,6 @@ int spz_batch_create(const spz_batch_instance* instances, size_t ninstances, con
       b->stall_for_test = true;
       b->wait_limit = 4096;
     }
-  }
-  if (b->tiles_per_item < 1) {
-    delete b;
-    return fail(SPZ_ERR_INVALID_ARGUMENT, "batch config: tiles_per_item must be >= 1");
   }
   if (b->kmax < 4 || b->kmax > kBatchMaxK || b->threads < 64 || b->threads > 1024 || (b->threads & 31)) {
     delete b;
