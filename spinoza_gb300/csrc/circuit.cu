@@ -28,6 +28,7 @@
 #include "gate_math.cuh"
 #include "tile_ops.cuh"
 #include "executor.cuh"
+#include "tile_fixed.cuh"
 
 namespace spz {
 
@@ -42,6 +43,7 @@ struct PassArgs {
   uint64_t ntiles;
   const TileGate* gates;
   const double2* tables;  // fast-mode phase tables (re, im)
+  const int4* fxtables;   // the same for fixed point: (re h, l, im h, l), see FlatTables; nullptr: FP64 only
   const int32_t* outcomes;  // device-side measurement outcomes (conditioned gates)
   int ngates;
   int k;            // local qubits
@@ -491,8 +493,8 @@ __device__ void tile_run_shfl(const PassArgs& A, uint64_t base, double* sre, dou
 // Every gate of the pass on one tile held in shared memory (sre, sim), in
 // pass order, with a block barrier after each (with SHFL, after each run of
 // warp-shuffle gates; without, runs are ignored and every gate is applied in
-// shared memory).
-template <bool SHFL>
+// shared memory).  FAST: the pass may hold fast-mode ops.
+template <bool SHFL, bool FAST>
 __device__ __forceinline__ void tile_pass_gates(const PassArgs& A, uint64_t base, double* sre, double* sim,
                                                 uint32_t T) {
   for (int gi = 0; gi < A.ngates; ++gi) {
@@ -516,10 +518,12 @@ __device__ __forceinline__ void tile_pass_gates(const PassArgs& A, uint64_t base
           case SPZ_GATE_Y: tile_pair_any<SPZ_GATE_Y, TileGate, TileSwizzle>(g, sre, sim, nw); break;
           case SPZ_GATE_RX: tile_pair_any<SPZ_GATE_RX, TileGate, TileSwizzle>(g, sre, sim, nw); break;
           case SPZ_GATE_RY: tile_pair_any<SPZ_GATE_RY, TileGate, TileSwizzle>(g, sre, sim, nw); break;
-#define SPZ_LAZY(FK)                                                            \
-  case FK:                                                                      \
-    if (g.pm) tile_fast_phase_pm<FK>(g, A.tables + g.ptab, base, sre, sim, nw); \
-    else tile_pair<FK, 1, TileGate, TileSwizzle>(g, sre, sim, nw);              \
+#define SPZ_LAZY(FK)                                                              \
+  case FK:                                                                        \
+    if constexpr (FAST) {                                                         \
+      if (g.pm) tile_fast_phase_pm<FK>(g, A.tables + g.ptab, base, sre, sim, nw); \
+      else tile_pair<FK, 1, TileGate, TileSwizzle>(g, sre, sim, nw);              \
+    }                                                                             \
     break;
           SPZ_LAZY(FK_LAZY_H)
           SPZ_LAZY(FK_LAZY_RX_A)
@@ -531,11 +535,13 @@ __device__ __forceinline__ void tile_pass_gates(const PassArgs& A, uint64_t base
         }
         break;
       case TM_PHASE:
-        if (g.npos) tile_phase_pm<1>(g, A.tables + g.ptab, base, sre, sim, nw);
-        else tile_phase_pm<0>(g, A.tables + g.ptab, base, sre, sim, nw);
+        if constexpr (FAST) {
+          if (g.npos) tile_phase_pm<1>(g, A.tables + g.ptab, base, sre, sim, nw);
+          else tile_phase_pm<0>(g, A.tables + g.ptab, base, sre, sim, nw);
+        }
         break;
       case TM_LAZY2:
-        tile_lazy2_pm(g, A.tables + g.ptab, base, sre, sim, nw);
+        if constexpr (FAST) tile_lazy2_pm(g, A.tables + g.ptab, base, sre, sim, nw);
         break;
       case TM_DIAG_LOCAL:
       case TM_DIAG_GLOBAL: {
@@ -558,8 +564,125 @@ __device__ __forceinline__ void tile_pass_gates(const PassArgs& A, uint64_t base
   }
 }
 
+// Every gate of the pass on one tile in fixed point, as tile_pass_gates.
 template <bool SHFL>
-__global__ void __launch_bounds__(kTileThreads, SHFL ? 12 : SPZ_TILE_MIN_BLOCKS) tile_kernel(PassArgs A) {
+__device__ __forceinline__ void fx_pass_gates(const PassArgs& A, uint64_t base, const FxTile& S, uint32_t T) {
+  for (int gi = 0; gi < A.ngates; ++gi) {
+    const TileGate& g = A.gates[gi];
+    if constexpr (SHFL) {
+      if (g.run_end > gi) {
+        for (uint32_t e = threadIdx.x; e < T; e += blockDim.x) {  // whole rows: T and blockDim are multiples of 32
+          FxAmp x = S.load(e);
+          for (int ri = gi; ri < g.run_end; ++ri) {
+            const TileGate& h = A.gates[ri];
+            if ((base & h.g_ones) != h.g_ones || (base & h.g_zeros) != 0) continue;
+            if (h.cond >= 0 && A.outcomes[h.cond] == 0) continue;
+            fx_run_gate(h, A.fxtables, base, e, x);
+          }
+          S.store(e, x);
+        }
+        gi = g.run_end - 1;
+        __syncthreads();
+        continue;
+      }
+    }
+    if ((base & g.g_ones) != g.g_ones || (base & g.g_zeros) != 0) continue;
+    if (g.cond >= 0 && A.outcomes[g.cond] == 0) continue;
+    if (g.mode == TM_DIAG_GLOBAL && g.kind != SPZ_GATE_RZ && !(base & g.g_tbit)) continue;
+    fx_tile_gate(g, A.fxtables, base, S, T);
+    __syncthreads();
+  }
+}
+
+// One tile between global and shared memory: `off` gives the global offset of
+// an even tile offset e (e and e + 1 are consecutive, 16-byte aligned).  In
+// shared memory they share a 16-byte slot too, in reverse order when the
+// swizzle flips the low bits.
+template <class Off>
+__device__ __forceinline__ void load_tile(const PassArgs& A, const Off& off, double* sre, double* sim, uint32_t T) {
+  for (uint32_t e2 = threadIdx.x; e2 < T / 2; e2 += blockDim.x) {
+    const uint32_t e = 2 * e2;
+    const uint64_t gi = off(e);
+    double2 r = *reinterpret_cast<const double2*>(A.re + gi);
+    double2 m = *reinterpret_cast<const double2*>(A.im + gi);
+    const uint32_t p = TileSwizzle::at(e) & ~1u;
+    if (p != e) {
+      r = make_double2(r.y, r.x);
+      m = make_double2(m.y, m.x);
+    }
+    *reinterpret_cast<double2*>(sre + p) = r;
+    *reinterpret_cast<double2*>(sim + p) = m;
+  }
+}
+
+template <class Off>
+__device__ __forceinline__ void store_tile(const PassArgs& A, const Off& off, const double* sre, const double* sim,
+                                           uint32_t T) {
+  for (uint32_t e2 = threadIdx.x; e2 < T / 2; e2 += blockDim.x) {
+    const uint32_t e = 2 * e2;
+    const uint64_t gi = off(e);
+    const uint32_t p = TileSwizzle::at(e) & ~1u;
+    double2 r = *reinterpret_cast<const double2*>(sre + p);
+    double2 m = *reinterpret_cast<const double2*>(sim + p);
+    if (p != e) {
+      r = make_double2(r.y, r.x);
+      m = make_double2(m.y, m.x);
+    }
+    *reinterpret_cast<double2*>(A.re + gi) = r;
+    *reinterpret_cast<double2*>(A.im + gi) = m;
+  }
+}
+
+// The pass on one tile in the fast mode.  The tile's FP64 amplitudes come from
+// global memory or, with `staged`, lie in shared memory already.  A tile of
+// zeros is left as it is (every op is linear); a tile that fixed point cannot
+// hold (fx_in_range) is worked on in FP64.
+template <bool SHFL, class Off>
+__device__ __forceinline__ void fast_tile(const PassArgs& A, uint64_t base, const Off& off, bool staged, double* sre,
+                                          double* sim, int32_t* sexp, uint32_t T) {
+  const FxTile S{reinterpret_cast<int64_t*>(sre), reinterpret_cast<int64_t*>(sim), sexp};
+  bool bad = A.fxtables == nullptr, any = false;
+  for (uint32_t e2 = threadIdx.x; e2 < T / 2; e2 += blockDim.x) {
+    const uint32_t e = 2 * e2;
+    double2 r, m;
+    if (staged) {
+      r = *reinterpret_cast<const double2*>(sre + e);
+      m = *reinterpret_cast<const double2*>(sim + e);
+    } else {
+      const uint64_t gi = off(e);
+      r = *reinterpret_cast<const double2*>(A.re + gi);
+      m = *reinterpret_cast<const double2*>(A.im + gi);
+    }
+    const uint64_t a = dbits(r.x), b = dbits(m.x), c = dbits(r.y), d = dbits(m.y);
+    bad |= !fx_in_range(a, b) || !fx_in_range(c, d);
+    any |= ((a | b | c | d) << 1) != 0;
+    const FxAmp x = fx_from(a, b), y = fx_from(c, d);
+    *reinterpret_cast<longlong2*>(S.r + e) = make_longlong2(x.r, y.r);
+    *reinterpret_cast<longlong2*>(S.i + e) = make_longlong2(x.i, y.i);
+    *reinterpret_cast<int2*>(S.e + e) = make_int2(x.e, y.e);
+  }
+  const int in_fp64 = __syncthreads_or(bad), nonzero = __syncthreads_or(any);
+  if (in_fp64) {
+    load_tile(A, off, sre, sim, T);
+    __syncthreads();
+    tile_pass_gates<SHFL, true>(A, base, sre, sim, T);
+    store_tile(A, off, sre, sim, T);
+    return;
+  }
+  if (!nonzero) return;
+  fx_pass_gates<SHFL>(A, base, S, T);
+  for (uint32_t e2 = threadIdx.x; e2 < T / 2; e2 += blockDim.x) {
+    const uint32_t e = 2 * e2;
+    const uint64_t gi = off(e);
+    const double2 x = fx_to_double(S.load(e)), y = fx_to_double(S.load(e + 1));
+    *reinterpret_cast<double2*>(A.re + gi) = make_double2(x.x, y.x);
+    *reinterpret_cast<double2*>(A.im + gi) = make_double2(x.y, y.y);
+  }
+}
+
+template <bool SHFL, bool FAST>
+__global__ void __launch_bounds__(kTileThreads, FAST ? SPZ_FAST_MIN_BLOCKS : SHFL ? 12 : SPZ_TILE_MIN_BLOCKS)
+    tile_kernel(PassArgs A) {
   extern __shared__ double smem[];
   const int K = A.k;
   const uint32_t T = 1u << K;
@@ -570,6 +693,7 @@ __global__ void __launch_bounds__(kTileThreads, SHFL ? 12 : SPZ_TILE_MIN_BLOCKS)
   // lets a 13th block of 2^10-amplitude tiles onto an SM.
   uint32_t* rowoff = reinterpret_cast<uint32_t*>(smem + 2 * T);
   const uint32_t nrows = 1u << A.nhigh;
+  int32_t* sexp = reinterpret_cast<int32_t*>(rowoff + (nrows + 1u & ~1u));  // FAST: the amplitudes' exponents
   const uint32_t cmask = (1u << A.c) - 1;
   // Row offsets: scatter of the high local bits, the same for every tile.
   // (The run-time index into A.lpos here and in deposit() keeps the parameter
@@ -586,37 +710,14 @@ __global__ void __launch_bounds__(kTileThreads, SHFL ? 12 : SPZ_TILE_MIN_BLOCKS)
   __syncthreads();
   for (uint64_t t = A.tile_begin + blockIdx.x; t < A.ntiles; t += gridDim.x) {
     const uint64_t base = deposit(slab_tile(A, t), A.lpos, K);
-    // load (pairs of consecutive amplitudes: c >= 1)
-    for (uint32_t e2 = threadIdx.x; e2 < T / 2; e2 += blockDim.x) {
-      const uint32_t e = 2 * e2;
-      const uint64_t gi = base | ((uint64_t)rowoff[e >> A.c] << A.c) | (e & cmask);
-      double2 r = *reinterpret_cast<const double2*>(A.re + gi);
-      double2 m = *reinterpret_cast<const double2*>(A.im + gi);
-      // e even: e and e + 1 share a 16-byte slot, in reverse order when the
-      // swizzle flips the low bits.
-      const uint32_t p = TileSwizzle::at(e) & ~1u;
-      if (p != e) {
-        r = make_double2(r.y, r.x);
-        m = make_double2(m.y, m.x);
-      }
-      *reinterpret_cast<double2*>(sre + p) = r;
-      *reinterpret_cast<double2*>(sim + p) = m;
-    }
-    __syncthreads();
-    tile_pass_gates<SHFL>(A, base, sre, sim, T);
-    // store
-    for (uint32_t e2 = threadIdx.x; e2 < T / 2; e2 += blockDim.x) {
-      const uint32_t e = 2 * e2;
-      const uint64_t gi = base | ((uint64_t)rowoff[e >> A.c] << A.c) | (e & cmask);
-      const uint32_t p = TileSwizzle::at(e) & ~1u;
-      double2 r = *reinterpret_cast<const double2*>(sre + p);
-      double2 m = *reinterpret_cast<const double2*>(sim + p);
-      if (p != e) {
-        r = make_double2(r.y, r.x);
-        m = make_double2(m.y, m.x);
-      }
-      *reinterpret_cast<double2*>(A.re + gi) = r;
-      *reinterpret_cast<double2*>(A.im + gi) = m;
+    const auto off = [&](uint32_t e) { return base | ((uint64_t)rowoff[e >> A.c] << A.c) | (e & cmask); };
+    if constexpr (FAST) {
+      fast_tile<SHFL>(A, base, off, false, sre, sim, sexp, T);
+    } else {
+      load_tile(A, off, sre, sim, T);
+      __syncthreads();
+      tile_pass_gates<SHFL, false>(A, base, sre, sim, T);
+      store_tile(A, off, sre, sim, T);
     }
     __syncthreads();
   }
@@ -680,7 +781,7 @@ __device__ __forceinline__ void tma_gather4(double* dst, const CUtensorMap* map,
       : "memory");
 }
 
-template <bool PREFETCH>
+template <bool PREFETCH, bool FAST>
 __global__ void __launch_bounds__(kTileThreads) tile_kernel_tma(PassArgs A, const __grid_constant__ CUtensorMap map_re,
                                                                 const __grid_constant__ CUtensorMap map_im, int* err) {
   extern __shared__ double smem_raw[];
@@ -747,12 +848,12 @@ __global__ void __launch_bounds__(kTileThreads) tile_kernel_tma(PassArgs A, cons
     double* sre = bufs + (size_t)b * 2 * T;
     double* sim = sre + T;
     const uint64_t base = deposit(tile, A.lpos, K);
-    tile_pass_gates<false>(A, base, sre, sim, T);
-    for (uint32_t e2 = threadIdx.x; e2 < T / 2; e2 += blockDim.x) {  // store, as the thread-load kernel
-      const uint32_t e = 2 * e2;
-      const uint64_t gi = base | rowoff[e >> kTileLowBits] | (e & ((1u << kTileLowBits) - 1));
-      *reinterpret_cast<double2*>(A.re + gi) = *reinterpret_cast<const double2*>(sre + e);
-      *reinterpret_cast<double2*>(A.im + gi) = *reinterpret_cast<const double2*>(sim + e);
+    const auto off = [&](uint32_t e) { return base | rowoff[e >> kTileLowBits] | (e & ((1u << kTileLowBits) - 1)); };
+    if constexpr (FAST) {
+      fast_tile<false>(A, base, off, true, sre, sim, reinterpret_cast<int32_t*>(rowoff + nrows), T);
+    } else {
+      tile_pass_gates<false, false>(A, base, sre, sim, T);
+      store_tile(A, off, sre, sim, T);
     }
     __syncthreads();
     if (!PREFETCH && next < A.ntiles) issue(next, 0);
@@ -858,6 +959,75 @@ std::vector<PlannedPass> plan(const std::vector<GateApp>& gates, uint32_t n, int
   return passes;
 }
 
+// A lazy op as its fixed-point form (tile_fixed.cuh): s1 times i^pre, the two
+// members swapped (swap), the rotation by t, then -1 on s0 (neg0) and i^post on
+// s1.  With s1' = i s1 an RX is an RY; the B forms are the A form with the
+// members swapped; H is the rotation by 1 after Z.
+struct FxLazy {
+  double t;
+  bool swap;
+  int pre, neg0, post;
+  uint32_t turns(int j) const { return (uint32_t)(j ? post : 2 * neg0) & 3u; }
+};
+
+FxLazy fx_lazy(int kind, double c) {
+  const bool neg = c < 0.0;
+  const double t = std::fabs(c);
+  switch (kind) {
+    case FK_LAZY_H: return FxLazy{1.0, false, 2, 0, 0};
+    case FK_LAZY_RY_A: return FxLazy{t, false, neg ? 2 : 0, 0, neg ? 2 : 0};
+    case FK_LAZY_RY_B: return FxLazy{t, true, neg ? 2 : 0, neg ? 0 : 1, 0};
+    case FK_LAZY_RX_A: return FxLazy{t, false, neg ? 3 : 1, 0, neg ? 1 : 3};
+    default: return FxLazy{t, true, neg ? 3 : 1, neg ? 0 : 1, 3};  // FK_LAZY_RX_B
+  }
+}
+
+// The phase tables of a run of passes as the kernels read them: entries (re,
+// im), and the same in fixed point, less the power of two of their table and
+// times the power of i that their lazy op starts with.
+struct FlatTables {
+  std::vector<double2> entries;
+  std::vector<int4> fixed;
+  bool finite = true;  // false: an angle was infinite or NaN, which fixed point cannot carry
+  void push(std::complex<double> w, int exponent, int turn) {
+    entries.push_back(make_double2(w.real(), w.imag()));
+    if (!std::isfinite(w.real()) || !std::isfinite(w.imag())) {
+      finite = false;
+      w = 0.0;
+    }
+    for (int j = 0; j < (turn & 3); ++j) w = std::complex<double>(-w.imag(), w.real());
+    const FxCoef x = fx_coef(std::ldexp(w.real(), -exponent)), y = fx_coef(std::ldexp(w.imag(), -exponent));
+    fixed.push_back(make_int4(x.h, x.l, y.h, y.l));
+  }
+  size_t bytes() const { return entries.size() * (sizeof(double2) + sizeof(int4)); }
+};
+
+// Entries of one table have one modulus (1, or the carried scale): the power
+// of two that brings it to (1/2, 1].  A modulus of 1 keeps 0.
+int table_exponent(const PhaseTable& t) {
+  const double mag = std::hypot(t.re[0], t.im[0]);
+  if (!(mag > 0.0) || !std::isfinite(mag) || (mag > 0.5 && mag < 1.0 + 1e-9)) return 0;
+  return std::ilogb(mag) + 1;
+}
+
+// Flatten `tables`; offsets[i] is the first entry of table i.
+FlatTables flatten(const std::vector<GateApp>& gates, const std::vector<PhaseTable>& tables,
+                   std::vector<uint32_t>* offsets) {
+  std::vector<int> turn(tables.size(), 0);
+  for (const GateApp& g : gates)
+    if (g.table >= 0 && g.kind != FK_PHASE) turn[g.table] = fx_lazy(g.kind, g.c.cs).pre;
+  FlatTables f;
+  for (const GateApp& g : gates)
+    if (g.kind >= FK_LAZY_H && g.kind <= FK_LAZY_RY_B && !std::isfinite(g.c.cs)) f.finite = false;
+  for (size_t k = 0; k < tables.size(); ++k) {
+    const PhaseTable& t = tables[k];
+    offsets->push_back((uint32_t)f.entries.size());
+    const int x = table_exponent(t);
+    for (size_t i = 0; i < t.re.size(); ++i) f.push({t.re[i], t.im[i]}, x, turn[k]);
+  }
+  return f;
+}
+
 // Build the device description of a gate inside a pass with local qubits `L`.
 TileGate tile_gate(const GateApp& g, const std::vector<int>& local, const std::vector<PhaseTable>* tables = nullptr,
                    const std::vector<uint32_t>* table_offsets = nullptr) {
@@ -868,6 +1038,12 @@ TileGate tile_gate(const GateApp& g, const std::vector<int>& local, const std::v
   t.kind = g.kind;
   t.c = g.c;
   t.cond = g.cond;
+  if (g.kind >= FK_LAZY_H && g.kind <= FK_LAZY_RY_B) {
+    const FxLazy x = fx_lazy(g.kind, g.c.cs);
+    t.fx1 = fx_coef(std::isfinite(x.t) ? x.t : 0.0);
+    t.fxswaps = x.swap ? 1u : 0u;
+    t.fxturns = x.turns(0) | (x.turns(1) << 2) | ((uint32_t)x.pre << 8);
+  }
   if (g.kind == FK_PHASE) {  // elementwise; any qubits (the global index is formed per amplitude)
     const PhaseTable& tab = (*tables)[g.table];
     t.mode = TM_PHASE;
@@ -879,6 +1055,7 @@ TileGate tile_gate(const GateApp& g, const std::vector<int>& local, const std::v
         if (((tab.mask[j] >> q) & 1) && where[q] >= 0) t.pemask[j] |= 1u << where[q];
     }
     t.ptab = (*table_offsets)[g.table];
+    t.fexp = table_exponent(tab);
     if (tab.half_bit) {
       // Only the half with the bit set is touched: a local bit is inserted into
       // the enumeration (every lane busy); a non-local one is a tile predicate.
@@ -1008,7 +1185,7 @@ size_t mark_shuffle_runs(TileGate* g, size_t count, int k) {
 // phase masks do not contain the first op's qubit (its phase then commutes
 // with the first rotation) and the two tables have at most kPhaseMaxTerms
 // masks between them.  pg[i] is the descriptor of gates[i]; the joint tables
-// are appended to `flat` (re, im pairs).  Returns the FP64 instructions
+// are appended to `flat`.  Returns the FP64 instructions
 // saved: 4 per block of four amplitudes, 2^n per fused pair.  SPZ_FAST_PAIRS=0
 // in the environment turns the fusion off (for A/B measurements).
 bool fast_pairs_enabled() {
@@ -1025,7 +1202,7 @@ bool lazy_with_table(const GateApp& g) {
 }
 
 uint64_t fuse_lazy_pairs(std::vector<TileGate>& pg, const std::vector<GateApp>& gates,
-                         const std::vector<PhaseTable>& tables, std::vector<double>* flat, uint32_t n) {
+                         const std::vector<PhaseTable>& tables, FlatTables* flat, uint32_t n) {
   if (!fast_pairs_enabled()) return 0;
   std::vector<TileGate> out;
   uint64_t saved = 0;
@@ -1045,6 +1222,11 @@ uint64_t fuse_lazy_pairs(std::vector<TileGate>& pg, const std::vector<GateApp>& 
         t.kind2 = u.kind;
         t.tbit2 = u.tbit;
         t.c.sn = u.c.cs;
+        const FxLazy x1 = fx_lazy(gates[i].kind, gates[i].c.cs), x2 = fx_lazy(gates[i + 1].kind, gates[i + 1].c.cs);
+        t.fx2 = u.fx1;
+        t.fxswaps = (x1.swap ? 1u : 0u) | (x2.swap ? 2u : 0u);
+        t.fxturns = 0;
+        for (int j = 0; j < 4; ++j) t.fxturns |= ((x1.turns(j & 1) + x2.turns(j >> 1)) & 3u) << (2 * j);
         const int p1 = __builtin_ctz(t.tbit), p2 = __builtin_ctz(u.tbit);
         t.npos = 2;
         t.pos[0] = (uint8_t)std::min(p1, p2);
@@ -1060,16 +1242,15 @@ uint64_t fuse_lazy_pairs(std::vector<TileGate>& pg, const std::vector<GateApp>& 
         uint32_t flip = 0;
         for (int j = 0; j < T1.m; ++j)
           if (T1.mask[j] & q2b) flip |= 1u << j;
-        t.ptab = (uint32_t)(flat->size() / 2);
+        t.ptab = (uint32_t)flat->entries.size();
         const uint32_t E = 1u << t.pm;
         for (uint32_t idx = 0; idx < E; ++idx) {
           const uint32_t i1 = idx & ((1u << T1.m) - 1), i2 = idx >> T1.m;
           const std::complex<double> w1(T1.re[i1], T1.im[i1]), w2(T2.re[i2], T2.im[i2]);
           const std::complex<double> w3 = std::complex<double>(T1.re[i1 ^ flip], T1.im[i1 ^ flip]) * w2;
-          for (const std::complex<double>& w : {w1, w2, w3}) {
-            flat->push_back(w.real());
-            flat->push_back(w.imag());
-          }
+          flat->push(w1, 0, x1.pre);
+          flat->push(w2, 0, x2.pre);
+          flat->push(w3, 0, x1.pre + x2.pre);
         }
         out.push_back(t);
         saved += 1ull << n;
@@ -1171,18 +1352,32 @@ uint64_t op_fp64_ops(uint32_t n, const GateApp& g, const std::vector<PhaseTable>
 // count; the grid of a tile pass is one wave of them (each block loops over
 // tiles), so no block waits for a second wave.  Cached per device and tile
 // size (kernel attributes are per device); callers may be on several threads.
-int tile_launch_shape(int device, int threads, size_t smem, int* resident_out, int* sms_out, bool shfl) {
+using TileKernel = void (*)(PassArgs);
+TileKernel tile_kernel_for(bool shfl, bool fast) {
+  if (fast) return shfl ? tile_kernel<true, true> : tile_kernel<false, true>;
+  return shfl ? tile_kernel<true, false> : tile_kernel<false, false>;
+}
+
+// Shared memory of a tile pass: the tile, the row table and, in the fast mode,
+// the amplitudes' exponents.
+size_t tile_smem(int k, int nhigh, bool fast) {
+  const size_t T = (size_t)1 << k, rows = (size_t)1 << nhigh;
+  return 2 * T * sizeof(double) + ((rows + 1) & ~(size_t)1) * sizeof(uint32_t) + (fast ? T * sizeof(int32_t) : 0);
+}
+
+int tile_launch_shape(int device, int threads, size_t smem, int* resident_out, int* sms_out, bool shfl, bool fast) {
   static std::mutex mu;
   static int sms[kMaxDevices] = {};
   // by log2 of the tile, 32 / 64 threads, and the instantiation
-  static int resident[kMaxDevices][kTileMaxK + 2][2][2] = {};
+  static int resident[kMaxDevices][kTileMaxK + 2][2][4] = {};
   if (device < 0 || device >= kMaxDevices) return fail(SPZ_ERR_INVALID_ARGUMENT, "device index out of range");
   std::lock_guard<std::mutex> lock(mu);
   if (!sms[device]) {
     int count = 0;
     SPZ_CUDA(cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, device));
-    const int max_smem = (2 << kTileMaxK) * 8 + (1 << (kTileMaxK - kTileLowBits)) * 8;
-    for (const void* fn : {(const void*)tile_kernel<false>, (const void*)tile_kernel<true>}) {
+    for (int v = 0; v < 4; ++v) {
+      const void* fn = (const void*)tile_kernel_for(v & 1, v & 2);
+      const int max_smem = (int)tile_smem(kTileMaxK, kTileMaxK - kTileLowBits, v & 2);
       SPZ_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
       SPZ_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout,
                                     cudaSharedmemCarveoutMaxShared));
@@ -1191,10 +1386,10 @@ int tile_launch_shape(int device, int threads, size_t smem, int* resident_out, i
   }
   int lg = 0;  // the largest lg with 2 x 8 B x 2^lg <= smem (the tile's re and im)
   while (lg <= kTileMaxK && (16ull << (lg + 1)) <= smem) ++lg;
-  int& r = resident[device][lg][threads > 32 ? 1 : 0][shfl ? 1 : 0];
+  int& r = resident[device][lg][threads > 32 ? 1 : 0][(shfl ? 1 : 0) + (fast ? 2 : 0)];
   if (!r) {
     int per_sm = 0;
-    const void* fn = shfl ? (const void*)tile_kernel<true> : (const void*)tile_kernel<false>;
+    const void* fn = (const void*)tile_kernel_for(shfl, fast);
     SPZ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem));
     r = std::max(1, per_sm);
   }
@@ -1241,15 +1436,22 @@ int ensure_tma_maps(spz_state_t h) {
 }
 
 // Blocks per SM of the TMA-staged kernel (per device and variant).
-int tma_launch_shape(int device, bool prefetch, int threads, size_t smem, int* resident_out) {
+using TmaKernel = void (*)(PassArgs, const CUtensorMap, const CUtensorMap, int*);
+TmaKernel tma_kernel_for(bool prefetch, bool fast) {
+  if (fast) return prefetch ? tile_kernel_tma<true, true> : tile_kernel_tma<false, true>;
+  return prefetch ? tile_kernel_tma<true, false> : tile_kernel_tma<false, false>;
+}
+
+int tma_launch_shape(int device, bool prefetch, bool fast, int threads, size_t smem, int* resident_out) {
   static std::mutex mu;
-  static int resident[kMaxDevices][2] = {};
+  static int resident[kMaxDevices][4] = {};
   if (device < 0 || device >= kMaxDevices) return fail(SPZ_ERR_INVALID_ARGUMENT, "device index out of range");
   std::lock_guard<std::mutex> lock(mu);
-  int& r = resident[device][prefetch];
+  int& r = resident[device][(prefetch ? 1 : 0) + (fast ? 2 : 0)];
   if (!r) {
-    const void* fn = prefetch ? (const void*)tile_kernel_tma<true> : (const void*)tile_kernel_tma<false>;
-    const int max_smem = (prefetch ? 4 : 2) * (8 << kTileMaxK) + (1 << (kTileMaxK - kTileLowBits)) * 8 + 128;
+    const void* fn = (const void*)tma_kernel_for(prefetch, fast);
+    const int max_smem = (prefetch ? 4 : 2) * (8 << kTileMaxK) + (1 << (kTileMaxK - kTileLowBits)) * 8 + 128 +
+                         (fast ? 4 << kTileMaxK : 0);
     SPZ_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
     SPZ_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
     int per_sm = 0;
@@ -1407,16 +1609,9 @@ int run_gates_io(spz_state_t h, const std::vector<GateApp>& gates_in, uint32_t f
   const int c = std::min<int>(kTileLowBits, k);
   std::vector<PlannedPass> passes = plan(gates, n, k, c, !fast);
   pad_tile_passes(passes, n, k);
-  // Phase tables, flattened (re, im) after the gate list.
+  // Phase tables, after the gate list.
   std::vector<uint32_t> table_offsets;
-  std::vector<double> flat;
-  for (const PhaseTable& t : tables) {
-    table_offsets.push_back((uint32_t)(flat.size() / 2));
-    for (size_t i = 0; i < t.re.size(); ++i) {
-      flat.push_back(t.re[i]);
-      flat.push_back(t.im[i]);
-    }
-  }
+  FlatTables flat = flatten(gates, tables, &table_offsets);
   // A pass runs as a tile pass unless it is one exact gate (the plain kernel
   // touches only what that gate needs); lowered fast ops exist only in tiles.
   auto tiled = [&](const PlannedPass& P) {
@@ -1443,19 +1638,24 @@ int run_gates_io(spz_state_t h, const std::vector<GateApp>& gates_in, uint32_t f
   }
   TileGate* dgates = nullptr;
   const double2* dtables = nullptr;
+  const int4* dfxtables = nullptr;
   if (!all.empty()) {
     void* dscr;
     const size_t gbytes = (all.size() * sizeof(TileGate) + 255) / 256 * 256;
-    const size_t tbytes = flat.size() * sizeof(double);
-    int rc = ensure_dev_scratch(h, gbytes + tbytes, &dscr);
+    const size_t tbytes = flat.entries.size() * sizeof(double2);
+    int rc = ensure_dev_scratch(h, gbytes + flat.bytes(), &dscr);
     if (rc) return rc;
     // From pageable memory: the runtime stages the bytes before returning, so
     // `all` and `flat` may go out of scope while the copies are still queued.
     SPZ_CUDA(cudaMemcpyAsync(dscr, all.data(), all.size() * sizeof(TileGate), cudaMemcpyHostToDevice, h->stream));
-    if (tbytes)
-      SPZ_CUDA(cudaMemcpyAsync((char*)dscr + gbytes, flat.data(), tbytes, cudaMemcpyHostToDevice, h->stream));
     dgates = (TileGate*)dscr;
     dtables = (const double2*)((char*)dscr + gbytes);
+    int4* fx = (int4*)((char*)dscr + gbytes + tbytes);
+    if (flat.finite) dfxtables = fx;
+    if (tbytes) {
+      SPZ_CUDA(cudaMemcpyAsync((void*)dtables, flat.entries.data(), tbytes, cudaMemcpyHostToDevice, h->stream));
+      SPZ_CUDA(cudaMemcpyAsync(fx, flat.fixed.data(), tbytes, cudaMemcpyHostToDevice, h->stream));
+    }
   }
 
   // TMA staging (SPZ_EXEC_TMA*): tensor maps once per handle; the timeout word
@@ -1513,33 +1713,33 @@ int run_gates_io(spz_state_t h, const std::vector<GateApp>& gates_in, uint32_t f
     }
     A.gates = dgates + offs[p];
     A.tables = dtables;
+    A.fxtables = dfxtables;
     A.outcomes = h->meas ? reinterpret_cast<const int32_t*>(h->meas + kMeasOutcomeOffset) : nullptr;
     A.ngates = (int)counts[p];
     const uint32_t T = 1u << A.k;
-    const size_t smem = 2 * T * sizeof(double) + (size_t)(1u << A.nhigh) * sizeof(uint32_t);
+    const size_t smem = tile_smem(A.k, A.nhigh, fast);
     const int threads = h->tile_threads ? h->tile_threads
                                         : (int)std::min<uint32_t>(kTileThreads, std::max<uint32_t>(32, T / 2));
     int resident = 0, sms = 0;
-    int rc = tile_launch_shape(h->device, threads, smem, &resident, &sms, shfl);
+    int rc = tile_launch_shape(h->device, threads, smem, &resident, &sms, shfl, fast);
     if (rc) return rc;
     if (use_tma && !A.slab_on && A.c == kTileLowBits && A.k >= kTileLowBits + 2) {
       const bool pre = (flags & SPZ_EXEC_TMA_PREFETCH) != 0;
-      const size_t tsmem = (pre ? 4 : 2) * T * sizeof(double) + (size_t)(1u << A.nhigh) * sizeof(uint64_t) + 128;
+      const size_t tsmem = (pre ? 4 : 2) * T * sizeof(double) + (size_t)(1u << A.nhigh) * sizeof(uint64_t) + 128 +
+                           (fast ? T * sizeof(int32_t) : 0);
       int tres = 0;
-      rc = tma_launch_shape(h->device, pre, threads, tsmem, &tres);
+      rc = tma_launch_shape(h->device, pre, fast, threads, tsmem, &tres);
       if (rc) return rc;
       CUtensorMap mre, mim;
       std::memcpy(&mre, h->tma_map[0], sizeof(mre));
       std::memcpy(&mim, h->tma_map[1], sizeof(mim));
       const uint64_t tblocks = std::min<uint64_t>(per, (uint64_t)sms * tres);
-      if (pre) tile_kernel_tma<true><<<(unsigned)tblocks, threads, tsmem, h->stream>>>(A, mre, mim, h->tma_err);
-      else tile_kernel_tma<false><<<(unsigned)tblocks, threads, tsmem, h->stream>>>(A, mre, mim, h->tma_err);
+      tma_kernel_for(pre, fast)<<<(unsigned)tblocks, threads, tsmem, h->stream>>>(A, mre, mim, h->tma_err);
       SPZ_CHECK_LAUNCH("tile_kernel_tma");
       return SPZ_OK;
     }
     const uint64_t blocks = std::min<uint64_t>(per, (uint64_t)sms * resident);
-    if (shfl) tile_kernel<true><<<(unsigned)blocks, threads, smem, h->stream>>>(A);
-    else tile_kernel<false><<<(unsigned)blocks, threads, smem, h->stream>>>(A);
+    tile_kernel_for(shfl, fast)<<<(unsigned)blocks, threads, smem, h->stream>>>(A);
     SPZ_CHECK_LAUNCH("tile_kernel");
     return SPZ_OK;
   };
@@ -1909,7 +2109,7 @@ int plan_stats(uint32_t n, const spz_op* ops, size_t nops, uint32_t flags, spz_e
       const std::vector<uint32_t> no_offsets(tables.size(), 0);
       std::vector<PlannedPass> planned = plan(run, n, k, c, !fast);
       pad_tile_passes(planned, n, k);
-      std::vector<double> no_flat;
+      FlatTables no_flat;
       for (const PlannedPass& P : planned) {
         const bool tiled = P.gates.size() > 1 || P.gates[0].kind >= FK_LAZY_H || P.gates[0].cond >= 0;
         size_t device_ops = P.gates.size();
@@ -1918,7 +2118,7 @@ int plan_stats(uint32_t n, const spz_op* ops, size_t nops, uint32_t flags, spz_e
           for (const GateApp& g : P.gates) tg.push_back(tile_gate(g, P.local, &tables, &no_offsets));
           if (fast) st->fp64_ops -= fuse_lazy_pairs(tg, P.gates, tables, &no_flat, n);
           if (flags & SPZ_EXEC_SHUFFLE) st->shuffle_gates += mark_shuffle_runs(tg.data(), tg.size(), (int)P.local.size());
-          no_flat.clear();
+          no_flat = FlatTables();
           device_ops = tg.size();
         }
         uint64_t L = 0;
@@ -1988,7 +2188,8 @@ struct ProgramPass {
   int threads = 0;
   size_t smem = 0;
   uint64_t blocks = 0;
-  bool shfl = false;   // tiled: launched as tile_kernel<true> (SPZ_EXEC_SHUFFLE)
+  bool shfl = false;   // tiled: with warp-shuffle runs (SPZ_EXEC_SHUFFLE)
+  bool fast = false;   // tiled: may hold fast-mode ops
 };
 
 }  // namespace spz
@@ -2057,14 +2258,7 @@ int build_program(spz_program_t p, const spz_op* ops, size_t nops, uint32_t flag
   std::vector<PlannedPass> planned = plan(gates, n, k, c, !fast);
   pad_tile_passes(planned, n, k);
   std::vector<uint32_t> table_offsets;
-  std::vector<double> flat;
-  for (const PhaseTable& t : tables) {
-    table_offsets.push_back((uint32_t)(flat.size() / 2));
-    for (size_t i = 0; i < t.re.size(); ++i) {
-      flat.push_back(t.re[i]);
-      flat.push_back(t.im[i]);
-    }
-  }
+  FlatTables flat = flatten(gates, tables, &table_offsets);
   std::vector<TileGate> all;
   std::vector<size_t> offs, counts;
   for (const PlannedPass& P : planned) {
@@ -2081,12 +2275,15 @@ int build_program(spz_program_t p, const spz_op* ops, size_t nops, uint32_t flag
     counts.push_back(pg.size());
   }
   const size_t gbytes = (all.size() * sizeof(TileGate) + 255) / 256 * 256;
-  const size_t tbytes = flat.size() * sizeof(double);
+  const size_t tbytes = flat.entries.size() * sizeof(double2);
   if (gbytes + tbytes) {
-    SPZ_CUDA(dev_alloc(&p->dbuf, gbytes + tbytes));
+    SPZ_CUDA(dev_alloc(&p->dbuf, gbytes + flat.bytes()));
     if (!all.empty())
       SPZ_CUDA(cudaMemcpy(p->dbuf, all.data(), all.size() * sizeof(TileGate), cudaMemcpyHostToDevice));
-    if (tbytes) SPZ_CUDA(cudaMemcpy((char*)p->dbuf + gbytes, flat.data(), tbytes, cudaMemcpyHostToDevice));
+    if (tbytes) {
+      SPZ_CUDA(cudaMemcpy((char*)p->dbuf + gbytes, flat.entries.data(), tbytes, cudaMemcpyHostToDevice));
+      SPZ_CUDA(cudaMemcpy((char*)p->dbuf + gbytes + tbytes, flat.fixed.data(), tbytes, cudaMemcpyHostToDevice));
+    }
   }
 
   for (size_t q = 0; q < planned.size(); ++q) {
@@ -2108,13 +2305,15 @@ int build_program(spz_program_t p, const spz_op* ops, size_t nops, uint32_t flag
     A.ntiles = 1ull << (n - A.k);
     A.gates = (const TileGate*)p->dbuf + offs[q];
     A.tables = (const double2*)((char*)p->dbuf + gbytes);
+    A.fxtables = flat.finite ? (const int4*)((char*)p->dbuf + gbytes + tbytes) : nullptr;
     A.ngates = (int)counts[q];
     const uint32_t T = 1u << A.k;
-    pp.smem = 2 * T * sizeof(double) + (size_t)(1u << A.nhigh) * sizeof(uint32_t);
+    pp.smem = tile_smem(A.k, A.nhigh, fast);
     pp.threads = (int)std::min<uint32_t>(kTileThreads, std::max<uint32_t>(32, T / 2));
     pp.shfl = (flags & SPZ_EXEC_SHUFFLE) != 0;
+    pp.fast = fast;
     int resident = 0, sms = 0;
-    int rc = tile_launch_shape(p->device, pp.threads, pp.smem, &resident, &sms, pp.shfl);
+    int rc = tile_launch_shape(p->device, pp.threads, pp.smem, &resident, &sms, pp.shfl, pp.fast);
     if (rc) return rc;
     pp.blocks = std::min<uint64_t>(A.ntiles, (uint64_t)sms * resident);
     p->stats.tile_passes++;
@@ -2145,8 +2344,7 @@ int capture_program(spz_program_t p, spz_state_t h) {
       A.re = h->re;
       A.im = h->im;
       A.outcomes = nullptr;
-      if (pp.shfl) tile_kernel<true><<<(unsigned)pp.blocks, pp.threads, pp.smem, p->capture>>>(A);
-      else tile_kernel<false><<<(unsigned)pp.blocks, pp.threads, pp.smem, p->capture>>>(A);
+      tile_kernel_for(pp.shfl, pp.fast)<<<(unsigned)pp.blocks, pp.threads, pp.smem, p->capture>>>(A);
       cudaError_t le = cudaGetLastError();
       if (le != cudaSuccess) rc = cuda_fail(le, "tile_kernel");
     }

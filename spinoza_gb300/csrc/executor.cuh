@@ -5,6 +5,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "fixed_point.cuh"
 
 namespace spz {
 
@@ -26,6 +27,9 @@ constexpr int kTileLowBits = 3;   // qubits 0..2 always local: 64-byte contiguou
 #endif
 #ifndef SPZ_TILE_MIN_BLOCKS
 #define SPZ_TILE_MIN_BLOCKS 13  // 13 x (16 KiB tile + 0.5 KiB row table + 1 KiB reserved) <= 228 KiB
+#endif
+#ifndef SPZ_FAST_MIN_BLOCKS
+#define SPZ_FAST_MIN_BLOCKS 10  // fast mode: 4 KiB of exponents more per tile
 #endif
 constexpr int kTileThreads = SPZ_TILE_THREADS;
 
@@ -63,6 +67,15 @@ struct TileGate {
   // SPZ_EXEC_SHUFFLE: > this gate's index, the end of a run of gates that the
   // block applies with warp shuffles (circuit.cu, tile_run_shfl); 0 otherwise.
   int32_t run_end;
+  // Fast mode in fixed point (tile_fixed.cuh).  A lazy op: its rotation's t
+  // (a TM_LAZY2's in fx1 and fx2), bit 0 / 1 of fxswaps: the two members are
+  // swapped before the first / second rotation, fxturns bits 2 j, 2 j + 1: the
+  // power of i that output j is multiplied by, bits 8, 9: the power of i on s1
+  // before the op (of a lazy op without a phase table; a table holds it in its
+  // entries).  A phase op: fexp, the power of two of its table.
+  FxCoef fx1, fx2;
+  uint32_t fxswaps, fxturns;
+  int32_t fexp;
 };
 
 // The descriptor of gate g inside a tile pass whose local qubits are `local`

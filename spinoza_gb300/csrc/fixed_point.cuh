@@ -1,0 +1,211 @@
+// Fast mode's arithmetic on the integer pipes: amplitudes in 64-bit fixed
+// point, each with an exponent of its own.
+//
+// What bounds the fast mode is DFMA issue (a warp's FP64 instruction holds the
+// SM's FP64 unit for 16 cycles), and its ops may round differently, so they
+// need no IEEE operation each.  For the length of a tile pass an amplitude is
+// (re, im) x 2^(exp - 1080): two 64-bit integers below 2^59 on one exponent.
+// An op brings the amplitudes that it mixes to the largest of their exponents;
+// a multiply-add by a coefficient of magnitude <= 1 is then four 32 x 32-bit
+// multiply-adds (1.3 cycles each), with no rounding, packing or normalising
+// between the ops of a pass.
+//
+// Precision: an op leaves an error of about 2^-58 of the largest amplitude
+// that it mixes, where FP64 rounds every operation to 2^-53 of its result.  The
+// amplitudes become FP64 again, rounded to nearest, when the pass stores them.
+// Tiles with a component that is not finite or a nonzero amplitude outside
+// [2^-895, 2^881) are worked on in FP64 (fx_in_range).
+//
+// Bounds.  An op's inputs have components below 2^59: a phase leaves them below
+// 2^59.5, a rotation below 2^60.5, a second one below 2^61.5; the limbs need
+// inputs below 2^61.  fx_shift then brings them below 2^59 again.
+#pragma once
+
+#include <math.h>
+#include <stdint.h>
+
+#ifdef __CUDACC__
+#define SPZ_HD __host__ __device__ __forceinline__
+#else
+#define SPZ_HD inline
+#endif
+
+namespace spz {
+
+constexpr uint32_t kFxMinHi = 0x08000000u;  // upper words of an amplitude's larger component: at least this ...
+constexpr uint32_t kFxMaxHi = 0x77000000u;  // ... and below this
+constexpr int kFxZeroExp = -(1 << 28);      // exponent of a zero amplitude
+
+struct FxAmp {
+  int64_t r, i;
+  int32_t e;
+};
+
+// A coefficient c, |c| <= 1 (and a rounding more), as (h 2^32 + l) / 2^62.
+struct FxCoef {
+  int32_t h, l;
+};
+
+inline FxCoef fx_coef(double c) {
+  const long long v = llrint(ldexp(c, 62));
+  const int32_t l = (int32_t)(uint32_t)(uint64_t)v;
+  return FxCoef{(int32_t)((v - l) >> 32), l};
+}
+
+// 4 y = h 2^32 + l, |y| < 2^61
+struct FxLimb {
+  int32_t h, l;
+};
+
+SPZ_HD FxLimb fx_split(int64_t y) {
+  const int32_t l = (int32_t)((uint32_t)y << 2);
+  return FxLimb{(int32_t)(y >> 30) + (int32_t)((uint32_t)l >> 31), l};
+}
+
+SPZ_HD int64_t fx_mad(int32_t a, int32_t b, int64_t c) { return (int64_t)a * b + c; }
+
+// x + c y = x + 4 y c 2^62 / 2^64: the products' low 32 bits are rounded away,
+// the product of the two low limbs (below the last bit) is left out.
+SPZ_HD int64_t fx_mac(int64_t x, const FxLimb& y, const FxCoef& c) {
+  const int64_t s = fx_mad(y.l, c.h, fx_mad(y.h, c.l, 1ll << 31));
+  return fx_mad(y.h, c.h, x) + (int32_t)(s >> 32);
+}
+
+// x - c y
+SPZ_HD int64_t fx_msub(int64_t x, const FxLimb& y, const FxCoef& c) {
+  const int64_t s = fx_mad(y.l, c.h, fx_mad(y.h, c.l, 1ll << 31));
+  return fx_mad(y.h, -c.h, x) - (int32_t)(s >> 32);
+}
+
+// (r, i) *= (x, y)
+SPZ_HD void fx_cmul(int64_t& r, int64_t& i, const FxCoef& x, const FxCoef& y) {
+  const FxLimb R = fx_split(r), I = fx_split(i);
+  const int64_t sr = fx_mad(R.l, x.h, fx_mad(R.h, x.l, 1ll << 31)), si = fx_mad(R.l, y.h, fx_mad(R.h, y.l, 1ll << 31));
+  const int64_t tr = fx_mad(I.l, -y.h, fx_mad(I.h, -y.l, sr)), ti = fx_mad(I.l, x.h, fx_mad(I.h, x.l, si));
+  r = fx_mad(I.h, -y.h, fx_mad(R.h, x.h, (int32_t)(tr >> 32)));
+  i = fx_mad(I.h, x.h, fx_mad(R.h, y.h, (int32_t)(ti >> 32)));
+}
+
+SPZ_HD int64_t fx_shr(int64_t v, int32_t d) {  // d >= 0, any size
+#ifdef __CUDA_ARCH__
+  int64_t r;
+  asm("shr.s64 %0, %1, %2;" : "=l"(r) : "l"(v), "r"(d));
+  return r;
+#else
+  return v >> (d < 63 ? d : 63);
+#endif
+}
+
+// The lazy rotation [[1, -t], [t, 1]] on s0, s1 with one exponent, 0 <= t <= 1.
+SPZ_HD void fx_rotate(FxAmp& s0, FxAmp& s1, const FxCoef& t) {
+  const FxLimb a = fx_split(s0.r), b = fx_split(s0.i), c = fx_split(s1.r), d = fx_split(s1.i);
+  s0.r = fx_msub(s0.r, c, t);
+  s0.i = fx_msub(s0.i, d, t);
+  s1.r = fx_mac(s1.r, a, t);
+  s1.i = fx_mac(s1.i, b, t);
+}
+
+// a *= i^p
+SPZ_HD void fx_quarter(FxAmp& a, uint32_t p) {
+  if (p & 2u) {
+    a.r = -a.r;
+    a.i = -a.i;
+  }
+  if (p & 1u) {
+    const int64_t r = a.r;
+    a.r = -a.i;
+    a.i = r;
+  }
+}
+
+SPZ_HD void fx_swap(FxAmp& a, FxAmp& b) {
+  const FxAmp t = a;
+  a = b;
+  b = t;
+}
+
+// Bring a[0 .. N-1] to the largest of their exponents, which is returned.
+template <int N>
+SPZ_HD int32_t fx_align(FxAmp* a) {
+  int32_t E = a[0].e;
+#pragma unroll
+  for (int j = 1; j < N; ++j) E = a[j].e > E ? a[j].e : E;
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    a[j].r = fx_shr(a[j].r, E - a[j].e);
+    a[j].i = fx_shr(a[j].i, E - a[j].e);
+  }
+  return E;
+}
+
+// Shift a[0 .. N-1], on exponent E, below 2^59 again.
+template <int N>
+SPZ_HD void fx_settle(FxAmp* a, int32_t E) {
+  uint32_t top = 0;
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    const int32_t r = (int32_t)(a[j].r >> 32), i = (int32_t)(a[j].i >> 32);
+    const uint32_t ar = (uint32_t)(r < 0 ? -r : r), ai = (uint32_t)(i < 0 ? -i : i);
+    top = ar > top ? ar : top;
+    top = ai > top ? ai : top;
+  }
+  if (top >= (1u << 27) - 1u) {  // |v| may reach 2^59 .. 2^61.5: 1 to 3 bits
+    const int32_t s = top < (1u << 28) - 1u ? 1 : top < (1u << 29) - 1u ? 2 : 3;
+    E += s;
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      a[j].r >>= s;
+      a[j].i >>= s;
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < N; ++j) a[j].e = E;
+}
+
+// The bits of an amplitude's components as FxAmp (any finite normal numbers; a
+// component far below the other, or subnormal, loses its low bits).
+SPZ_HD FxAmp fx_from(uint64_t re, uint64_t im) {
+  const uint32_t hr = (uint32_t)(re >> 32) & 0x7FFFFFFFu, hi = (uint32_t)(im >> 32) & 0x7FFFFFFFu;
+  const int32_t e = (int32_t)((hr > hi ? hr : hi) >> 20);
+  int64_t v[2];
+  const uint64_t b[2] = {re, im};
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const uint32_t h = (uint32_t)(b[j] >> 32);
+    const uint64_t m = (((uint64_t)((h & 0x000FFFFFu) | 0x00100000u) << 32) | (uint32_t)b[j]) << 5;
+    const int32_t f = (int32_t)((h >> 20) & 0x7FFu);
+    const int64_t s = (int64_t)((int32_t)h >> 31);
+    v[j] = f == 0 ? 0 : ((fx_shr((int64_t)m, e - f) ^ s) - s);
+  }
+  return FxAmp{v[0], v[1], e == 0 ? kFxZeroExp : e};
+}
+
+// Whether fx_from keeps the amplitude (zero, or its larger component in range).
+SPZ_HD bool fx_in_range(uint64_t re, uint64_t im) {
+  const uint32_t hr = (uint32_t)(re >> 32) & 0x7FFFFFFFu, hi = (uint32_t)(im >> 32) & 0x7FFFFFFFu;
+  const uint32_t big = hr > hi ? hr : hi;
+  return big - kFxMinHi < kFxMaxHi - kFxMinHi || ((re | im) << 1) == 0;
+}
+
+// v 2^(E - 1080) as FP64 bits, rounded to nearest, for 64 <= E < 1980.
+SPZ_HD uint64_t fx_bits(int64_t v, int32_t E) {
+  const int64_t s = v >> 63;
+  const uint64_t a = (uint64_t)((v ^ s) - s);
+#ifdef __CUDA_ARCH__
+  // the exponent of a: its upper and lower half rounded toward zero to FP32
+  const uint32_t ah = (uint32_t)(a >> 32), al = (uint32_t)a;
+  const uint32_t q = __float_as_uint(__fmaf_rz(__uint2float_rz(ah), 4294967296.0f, __uint2float_rz(al))) >> 23;
+  uint64_t n;
+  asm("shl.b64 %0, %1, %2;" : "=l"(n) : "l"(a), "r"(189u - q));  // leading one to bit 62 (0 for a = 0)
+#else
+  const uint32_t q = a ? 127u + 63u - (uint32_t)__builtin_clzll(a) : 0u;
+  const uint64_t n = a ? a << (189u - q) : 0;
+#endif
+  const uint64_t m = (n + 0x200u) >> 10;
+  uint32_t hi = (uint32_t)(m >> 32) + ((q + (uint32_t)(E - 185)) << 20);  // E + (q - 127 - 57) - 1
+  hi |= (uint32_t)s & 0x80000000u;
+  hi = a ? hi : 0u;
+  return ((uint64_t)hi << 32) | (uint32_t)m;
+}
+
+}  // namespace spz

@@ -14,6 +14,8 @@ namespace spz {
 
 constexpr double kSqrtOneHalf = 0.70710678118654752440;  // math.rs:5
 
+__device__ __forceinline__ uint64_t dbits(double a) { return (uint64_t)__double_as_longlong(a); }
+
 // Fast-mode lazy ops (the gate divided by a scalar carried elsewhere): four
 // FP64 instructions per pair.  Coefficient in g.cs (t or u).
 template <int FK>
@@ -56,7 +58,6 @@ __device__ __forceinline__ void fast_pair_kind(int kind, double t, double& a, do
 // qubits, H + RX + RZ + U + CX + 3-control X on every target: 159.1 ms with
 // DFMA products, 109.7 with six of a rotation's eight moved, 107.5 with eight;
 // 26-qubit exact brickwork 226.4 -> 177.5 ms).
-__device__ __forceinline__ uint64_t dbits(double a) { return (uint64_t)__double_as_longlong(a); }
 __device__ __forceinline__ double imul(double y, const MulCoef& c) {
   return __longlong_as_double((long long)mul_int(dbits(y), c));
 }
