@@ -29,6 +29,7 @@
 #include "tile_ops.cuh"
 #include "executor.cuh"
 #include "tile_fixed.cuh"
+#include "tile_map.cuh"
 
 namespace spz {
 
@@ -66,218 +67,102 @@ __device__ __forceinline__ uint64_t slab_tile(const PassArgs& A, uint64_t t) {
 }
 
 // ------------------------------------------------------------ device side
-// Nibble-swizzled tile layout: removes the 2-way bank conflicts of pair ops on
-// tile bits 0-3, but measured no faster on the 30-qubit brickwork (the passes
-// are DFMA-bound, not shared-memory bound), so off by default.
-#ifndef SPZ_TILE_SWIZZLE
-#define SPZ_TILE_SWIZZLE 0
-#endif
-#if SPZ_TILE_SWIZZLE
-using TileSwizzle = NibbleSwizzle;  // tile layout in shared memory (tile_ops.cuh)
-#else
-using TileSwizzle = NoSwizzle;
-#endif
-
-// Lazy op with its phase: s1 *= table[parities], then the lazy rotation.  Lazy
-// ops are uncontrolled, so the target is the only inserted position.  The
-// masks exclude the target, so both members of a pair share the entry.  (The
-// tables, 2-8 entries in a brickwork, are read through L1; holding them one
-// entry per lane and reading them with warp shuffles measured 1.2% slower.)
-template <int FK, int PM>
-__device__ __forceinline__ void tile_fast_phase(const TileGate& g, const double2* __restrict__ tab, uint64_t base,
-                                                double* sre, double* sim, uint32_t npairs) {
-  const Enumerator<1, TileGate> E(g);
-  const uint32_t tbit = g.tbit;
-  const Coef c = g.c;
-  uint32_t em[PM];
-  uint32_t bidx = 0;
-#pragma unroll
-  for (int j = 0; j < PM; ++j) {
-    bidx |= (uint32_t)(__popcll(base & g.pmask[j]) & 1) << j;
-    em[j] = g.pemask[j];
-  }
-  if constexpr (kTileBatch > 1) {  // see tile_pair
-    const uint32_t step = blockDim.x;
-    for (uint32_t m0 = threadIdx.x; m0 < npairs; m0 += kTileBatch * step) {
-      uint32_t s0[kTileBatch], s1[kTileBatch];
-      double a[kTileBatch], b[kTileBatch], x[kTileBatch], d[kTileBatch];
-      double2 w[kTileBatch];
-#pragma unroll
-      for (int u = 0; u < kTileBatch; ++u) {
-        const uint32_t m = m0 + u * step;
-        const uint32_t e0 = E(m < npairs ? m : m0);
-        s0[u] = TileSwizzle::at(e0);
-        s1[u] = TileSwizzle::at(e0 | tbit);
-        uint32_t idx = bidx;
-#pragma unroll
-        for (int j = 0; j < PM; ++j) idx ^= (uint32_t)(__popc(e0 & em[j]) & 1) << j;
-        w[u] = __ldg(tab + idx);
-        a[u] = sre[s0[u]]; b[u] = sim[s0[u]]; x[u] = sre[s1[u]]; d[u] = sim[s1[u]];
-      }
-#pragma unroll
-      for (int u = 0; u < kTileBatch; ++u) {
-        const double r = x[u], i = d[u];
-        x[u] = dfma(r, w[u].x, dmul(dneg(i), w[u].y));
-        d[u] = dfma(r, w[u].y, dmul(i, w[u].x));
-        fast_pair<FK>(c, a[u], b[u], x[u], d[u]);
-      }
-#pragma unroll
-      for (int u = 0; u < kTileBatch; ++u) {
-        if (m0 + u * step < npairs) {
-          sre[s0[u]] = a[u]; sim[s0[u]] = b[u]; sre[s1[u]] = x[u]; sim[s1[u]] = d[u];
-        }
-      }
-    }
-  } else {
-#pragma unroll kTileUnroll
-    for (uint32_t m = threadIdx.x; m < npairs; m += blockDim.x) {
-      const uint32_t e0 = E(m);
-      const uint32_t s0 = TileSwizzle::at(e0), s1 = TileSwizzle::at(e0 | tbit);
-      uint32_t idx = bidx;
-#pragma unroll
-      for (int j = 0; j < PM; ++j) idx ^= (uint32_t)(__popc(e0 & em[j]) & 1) << j;
-      const double2 w = __ldg(tab + idx);
-      double a = sre[s0], b = sim[s0];
-      const double r = sre[s1], i = sim[s1];
-      double x = dfma(r, w.x, dmul(dneg(i), w.y));
-      double d = dfma(r, w.y, dmul(i, w.x));
-      fast_pair<FK>(c, a, b, x, d);
-      sre[s0] = a; sim[s0] = b; sre[s1] = x; sim[s1] = d;
-    }
+// FP64 ops on a tile.  Items, slots and phase indices come from the op's walk
+// (tile_map.cuh); one thread works on a pair, an amplitude or a block of four
+// at a time.
+template <int KIND>
+__device__ __forceinline__ void tile_pair_op(const TileGate& g, Walk W, double* sre, double* sim, uint32_t n) {
+  const PairGate<KIND> op(g.c);
+  const uint32_t tmask = g.tmask;
+  for (uint32_t m = threadIdx.x, it = 0; m < n; m += blockDim.x, ++it) {
+    const uint32_t s0 = W.word(it), s1 = s0 ^ tmask;
+    double a = sre[s0], b = sim[s0], c = sre[s1], d = sim[s1];
+    op(a, b, c, d);
+    sre[s0] = a; sim[s0] = b; sre[s1] = c; sim[s1] = d;
   }
 }
 
-template <int FK>
-__device__ __forceinline__ void tile_fast_phase_pm(const TileGate& g, const double2* tab, uint64_t base, double* sre,
-                                                   double* sim, uint32_t npairs) {
-  switch (g.pm) {
-    case 1: tile_fast_phase<FK, 1>(g, tab, base, sre, sim, npairs); break;
-    case 2: tile_fast_phase<FK, 2>(g, tab, base, sre, sim, npairs); break;
-    case 3: tile_fast_phase<FK, 3>(g, tab, base, sre, sim, npairs); break;
-    case 4: tile_fast_phase<FK, 4>(g, tab, base, sre, sim, npairs); break;
-    case 5: tile_fast_phase<FK, 5>(g, tab, base, sre, sim, npairs); break;
-    case 6: tile_fast_phase<FK, 6>(g, tab, base, sre, sim, npairs); break;
-    case 7: tile_fast_phase<FK, 7>(g, tab, base, sre, sim, npairs); break;
-    default: tile_fast_phase<FK, kPhaseMaxTerms>(g, tab, base, sre, sim, npairs); break;
+template <int KIND>
+__device__ __forceinline__ void tile_diag_op(const TileGate& g, Walk W, double* sre, double* sim, uint32_t n,
+                                             int global_one) {
+  const DiagGate<KIND> op(g.d);
+  for (uint32_t m = threadIdx.x, it = 0; m < n; m += blockDim.x, ++it) {
+    const uint32_t w = W.word(it), s = w & 0xFFFFu;
+    double r = sre[s], i = sim[s];
+    op(global_one >= 0 ? global_one != 0 : (w >> 16) != 0, r, i);
+    sre[s] = r; sim[s] = i;
   }
 }
 
-// Fast-mode phase op: per amplitude, a table entry chosen by index parities.
-// The amplitudes visited are the tile's (npos = 0) or, for a local half bit,
-// those with that bit set (inserted by the enumeration).
-// parity(x & mask) = parity(base & mask) ^ parity(e & local part of mask); the
-// first is uniform over the tile.
-template <int NPOS, int PM>
-__device__ __forceinline__ void tile_phase(const TileGate& g, const double2* __restrict__ tab, uint64_t base,
-                                           double* sre, double* sim, uint32_t nelem) {
-  const Enumerator<NPOS, TileGate> E(g);
-  uint32_t em[PM > 0 ? PM : 1];
-  uint32_t bidx = 0;
-#pragma unroll
-  for (int j = 0; j < PM; ++j) {
-    bidx |= (uint32_t)(__popcll(base & g.pmask[j]) & 1) << j;
-    em[j] = g.pemask[j];
-  }
-#pragma unroll kTileUnroll
-  for (uint32_t m = threadIdx.x; m < nelem; m += blockDim.x) {
-    const uint32_t e0 = E(m);
-    uint32_t idx = bidx;
-#pragma unroll
-    for (int j = 0; j < PM; ++j) idx ^= (uint32_t)(__popc(e0 & em[j]) & 1) << j;
-    const uint32_t e = TileSwizzle::at(e0);
-    const double2 w = __ldg(tab + idx);
-    const double r = sre[e], i = sim[e];
-    sre[e] = dfma(r, w.x, dmul(dneg(i), w.y));
-    sim[e] = dfma(r, w.y, dmul(i, w.x));
+__device__ __forceinline__ void tile_swap_op(const TileGate& g, Walk W, double* sre, double* sim, uint32_t n) {
+  const uint32_t t1 = g.tmask, t2 = g.tmask2;
+  for (uint32_t m = threadIdx.x, it = 0; m < n; m += blockDim.x, ++it) {
+    const uint32_t b = W.word(it), i = b ^ t2, j = b ^ t1;
+    const double r = sre[i], q = sim[i];
+    sre[i] = sre[j]; sim[i] = sim[j];
+    sre[j] = r; sim[j] = q;
   }
 }
 
-template <int NPOS>
-__device__ __forceinline__ void tile_phase_pm(const TileGate& g, const double2* tab, uint64_t base, double* sre,
-                                              double* sim, uint32_t nelem) {
-  switch (g.pm) {
-    case 0: tile_phase<NPOS, 0>(g, tab, base, sre, sim, nelem); break;
-    case 1: tile_phase<NPOS, 1>(g, tab, base, sre, sim, nelem); break;
-    case 2: tile_phase<NPOS, 2>(g, tab, base, sre, sim, nelem); break;
-    case 3: tile_phase<NPOS, 3>(g, tab, base, sre, sim, nelem); break;
-    case 4: tile_phase<NPOS, 4>(g, tab, base, sre, sim, nelem); break;
-    case 5: tile_phase<NPOS, 5>(g, tab, base, sre, sim, nelem); break;
-    case 6: tile_phase<NPOS, 6>(g, tab, base, sre, sim, nelem); break;
-    case 7: tile_phase<NPOS, 7>(g, tab, base, sre, sim, nelem); break;
-    default: tile_phase<NPOS, kPhaseMaxTerms>(g, tab, base, sre, sim, nelem); break;
+// Fast-mode ops in FP64, for the tiles that fixed point cannot hold (the fast
+// mode's own code is tile_fixed.cuh).
+__device__ __forceinline__ void phase_mul(const double2& w, double& r, double& i) {
+  const double x = r, y = i;
+  r = dfma(x, w.x, dmul(dneg(y), w.y));
+  i = dfma(x, w.y, dmul(y, w.x));
+}
+
+// Lazy op, s1 first multiplied by its phase entry when the op has a table.
+static __device__ void tile_lazy_op(const TileGate& g, Walk W, const double2* __restrict__ tab, double* sre,
+                                    double* sim, uint32_t n) {
+  const uint32_t tmask = g.tmask;
+  for (uint32_t m = threadIdx.x, it = 0; m < n; m += blockDim.x, ++it) {
+    const uint32_t w = W.word(it), s0 = w & 0xFFFFu, s1 = s0 ^ tmask;
+    double a = sre[s0], b = sim[s0], c = sre[s1], d = sim[s1];
+    if (g.pm) phase_mul(__ldg(tab + (w >> 16)), c, d);
+    fast_pair_kind(g.kind, g.c.cs, a, b, c, d);
+    sre[s0] = a; sim[s0] = b; sre[s1] = c; sim[s1] = d;
   }
 }
 
-// Fast mode, two lazy rotations fused (TM_LAZY2): on each block of four
-// amplitudes (tile bits b1 = tbit, b2 = tbit2), the first op's phase on the
-// b1 = 1 half and the second op's phase on the b2 = 1 half are applied
-// together (the second op's phase masks never contain the first op's qubit,
-// so it commutes with the first rotation): three complex multiplies by one
-// table row instead of four, then the first rotation on the two pairs along
-// b1 and the second on the two pairs along b2.  28 FP64 instructions per
-// block instead of 32, one shared-memory round trip and one barrier for both.
-template <int PM>
-__device__ __forceinline__ void tile_lazy2(const TileGate& g, const double2* __restrict__ tab, uint64_t base,
-                                           double* sre, double* sim, uint32_t nblocks) {
-  const Enumerator<2, TileGate> E(g);
-  const uint32_t b1 = g.tbit, b2 = g.tbit2;
-  const double t1 = g.c.cs, t2 = g.c.sn;
-  const int k1 = g.kind, k2 = g.kind2;
-  uint32_t em[PM > 0 ? PM : 1];
-  uint32_t bidx = 0;
-#pragma unroll
-  for (int j = 0; j < PM; ++j) {
-    if (j < g.pm) {
-      bidx |= (uint32_t)(__popcll(base & g.pmask[j]) & 1) << j;
-      em[j] = g.pemask[j];
-    } else {
-      em[j] = 0;
-    }
+static __device__ void tile_phase_op(Walk W, const double2* __restrict__ tab, double* sre, double* sim,
+                                     uint32_t n) {
+  for (uint32_t m = threadIdx.x, it = 0; m < n; m += blockDim.x, ++it) {
+    const uint32_t w = W.word(it), s = w & 0xFFFFu;
+    double r = sre[s], i = sim[s];
+    phase_mul(__ldg(tab + (w >> 16)), r, i);
+    sre[s] = r; sim[s] = i;
   }
-  for (uint32_t m = threadIdx.x; m < nblocks; m += blockDim.x) {
-    const uint32_t e = E(m);
-    uint32_t idx = bidx;
-#pragma unroll
-    for (int j = 0; j < PM; ++j) idx ^= (uint32_t)(__popc(e & em[j]) & 1) << j;
-    const double2* row = tab + 3 * idx;
-    const uint32_t e1 = TileSwizzle::at(e | b1), e2 = TileSwizzle::at(e | b2), e3 = TileSwizzle::at(e | b1 | b2);
-    const uint32_t e0 = TileSwizzle::at(e);
+}
+
+// Two lazy rotations fused (TM_LAZY2): on each block of four amplitudes (tile
+// bits b1 = tbit, b2 = tbit2), the first op's phase on the b1 = 1 half and the
+// second op's phase on the b2 = 1 half are applied together (the second op's
+// phase masks never contain the first op's qubit, so it commutes with the
+// first rotation): three complex multiplies by one table row instead of four,
+// then the first rotation on the two pairs along b1 and the second on the two
+// pairs along b2.
+static __device__ void tile_lazy2_op(const TileGate& g, Walk W, const double2* __restrict__ tab, double* sre,
+                                     double* sim, uint32_t n) {
+  const uint32_t b1 = g.tmask, b2 = g.tmask2;
+  for (uint32_t m = threadIdx.x, it = 0; m < n; m += blockDim.x, ++it) {
+    const uint32_t w = W.word(it), e0 = w & 0xFFFFu, e1 = e0 ^ b1, e2 = e0 ^ b2, e3 = e1 ^ b2;
+    const double2* row = tab + 3 * (w >> 16);
     double r0 = sre[e0], i0 = sim[e0];
     double r1 = sre[e1], i1 = sim[e1];
     double r2 = sre[e2], i2 = sim[e2];
     double r3 = sre[e3], i3 = sim[e3];
-    {
-      const double2 w1 = __ldg(row), w2 = __ldg(row + 1), w3 = __ldg(row + 2);
-      double x = r1, y = i1;
-      r1 = dfma(x, w1.x, dmul(dneg(y), w1.y));
-      i1 = dfma(x, w1.y, dmul(y, w1.x));
-      x = r2; y = i2;
-      r2 = dfma(x, w2.x, dmul(dneg(y), w2.y));
-      i2 = dfma(x, w2.y, dmul(y, w2.x));
-      x = r3; y = i3;
-      r3 = dfma(x, w3.x, dmul(dneg(y), w3.y));
-      i3 = dfma(x, w3.y, dmul(y, w3.x));
-    }
-    fast_pair_kind(k1, t1, r0, i0, r1, i1);  // along b1
-    fast_pair_kind(k1, t1, r2, i2, r3, i3);
-    fast_pair_kind(k2, t2, r0, i0, r2, i2);  // along b2
-    fast_pair_kind(k2, t2, r1, i1, r3, i3);
+    phase_mul(__ldg(row), r1, i1);
+    phase_mul(__ldg(row + 1), r2, i2);
+    phase_mul(__ldg(row + 2), r3, i3);
+    fast_pair_kind(g.kind, g.c.cs, r0, i0, r1, i1);  // along b1
+    fast_pair_kind(g.kind, g.c.cs, r2, i2, r3, i3);
+    fast_pair_kind(g.kind2, g.c.sn, r0, i0, r2, i2);  // along b2
+    fast_pair_kind(g.kind2, g.c.sn, r1, i1, r3, i3);
     sre[e0] = r0; sim[e0] = i0;
     sre[e1] = r1; sim[e1] = i1;
     sre[e2] = r2; sim[e2] = i2;
     sre[e3] = r3; sim[e3] = i3;
-  }
-}
-
-__device__ __forceinline__ void tile_lazy2_pm(const TileGate& g, const double2* tab, uint64_t base, double* sre,
-                                              double* sim, uint32_t nblocks) {
-  switch (g.pm) {
-    case 2: tile_lazy2<2>(g, tab, base, sre, sim, nblocks); break;
-    case 3: tile_lazy2<3>(g, tab, base, sre, sim, nblocks); break;
-    case 4: tile_lazy2<4>(g, tab, base, sre, sim, nblocks); break;
-    case 5: tile_lazy2<5>(g, tab, base, sre, sim, nblocks); break;
-    case 6: tile_lazy2<6>(g, tab, base, sre, sim, nblocks); break;
-    default: tile_lazy2<kPhaseMaxTerms>(g, tab, base, sre, sim, nblocks); break;
   }
 }
 
@@ -304,10 +189,8 @@ __device__ __forceinline__ uint32_t phase_index(const TileGate& g, uint64_t base
   return idx;
 }
 
-// Lazy op of a run: the descriptor's phase masks are read once per row group
-// into registers (PM of them; the table index of an amplitude is the tile's
-// parities xor the local ones).
-template <int R, int PM>
+// Lazy op of a run.
+template <int R>
 __device__ __forceinline__ void run_lazy(const TileGate& g, const double2* __restrict__ tables, uint64_t base,
                                          uint32_t lane, const uint32_t* e, double* xr, double* xi) {
   const uint32_t tb = g.tbit;
@@ -315,25 +198,11 @@ __device__ __forceinline__ void run_lazy(const TileGate& g, const double2* __res
   const int kind = g.kind;
   const double t = g.c.cs;
   const double2* tab = tables + g.ptab;
-  uint32_t em[PM > 0 ? PM : 1];
-  uint32_t bidx = 0;
-#pragma unroll
-  for (int j = 0; j < PM; ++j) {
-    if (j < g.pm) {
-      bidx |= (uint32_t)(__popcll(base & g.pmask[j]) & 1) << j;
-      em[j] = g.pemask[j];
-    } else {
-      em[j] = 0;
-    }
-  }
 #pragma unroll
   for (int u = 0; u < R; ++u) {
     double pr = shfl_x(xr[u], tb), pi = shfl_x(xi[u], tb);
-    if constexpr (PM > 0) {  // s1 x w: the s1 lane forms the real part, the s0 lane the imaginary part
-      uint32_t idx = bidx;
-#pragma unroll
-      for (int j = 0; j < PM; ++j) idx ^= (uint32_t)(__popc(e[u] & em[j]) & 1) << j;
-      const double2 w = __ldg(tab + idx);
+    if (g.pm > 0) {  // s1 x w: the s1 lane forms the real part, the s0 lane the imaginary part
+      const double2 w = __ldg(tab + phase_index(g, base, e[u]));
       const double r = hi ? xr[u] : pr, i = hi ? xi[u] : pi;
       const double v = dfma(r, hi ? w.x : w.y, dmul(hi ? dneg(i) : i, hi ? w.y : w.x));
       const double vp = shfl_x(v, tb);
@@ -415,14 +284,7 @@ __device__ __forceinline__ void run_pair(const TileGate& g, const double2* __res
       xi[u] = dfma(1.0, pi, tp);
     }
   } else {  // fast-mode lazy ops, s1 first multiplied by its phase entry when the op carries one
-    switch (g.pm) {
-      case 0: run_lazy<R, 0>(g, tables, base, lane, e, xr, xi); break;
-      case 1: run_lazy<R, 1>(g, tables, base, lane, e, xr, xi); break;
-      case 2: run_lazy<R, 2>(g, tables, base, lane, e, xr, xi); break;
-      case 3: run_lazy<R, 3>(g, tables, base, lane, e, xr, xi); break;
-      case 4: run_lazy<R, 4>(g, tables, base, lane, e, xr, xi); break;
-      default: run_lazy<R, kPhaseMaxTerms>(g, tables, base, lane, e, xr, xi); break;
-    }
+    run_lazy<R>(g, tables, base, lane, e, xr, xi);
   }
 }
 
@@ -472,8 +334,8 @@ __device__ void tile_run_shfl(const PassArgs& A, uint64_t base, double* sre, dou
 #pragma unroll
     for (int u = 0; u < R; ++u) {
       e[u] = ((r0 + u) << 5) | lane;
-      xr[u] = sre[TileSwizzle::at(e[u])];
-      xi[u] = sim[TileSwizzle::at(e[u])];
+      xr[u] = sre[e[u]];
+      xi[u] = sim[e[u]];
     }
     for (int gi = g0; gi < g1; ++gi) {
       const TileGate& g = A.gates[gi];
@@ -484,19 +346,20 @@ __device__ void tile_run_shfl(const PassArgs& A, uint64_t base, double* sre, dou
     }
 #pragma unroll
     for (int u = 0; u < R; ++u) {
-      sre[TileSwizzle::at(e[u])] = xr[u];
-      sim[TileSwizzle::at(e[u])] = xi[u];
+      sre[e[u]] = xr[u];
+      sim[e[u]] = xi[u];
     }
   }
 }
 
 // Every gate of the pass on one tile held in shared memory (sre, sim), in
-// pass order, with a block barrier after each (with SHFL, after each run of
-// warp-shuffle gates; without, runs are ignored and every gate is applied in
-// shared memory).  FAST: the pass may hold fast-mode ops.
+// pass order, with a block barrier after each that works on amplitudes (with
+// SHFL, after each run of warp-shuffle gates; without, runs are ignored).
+// FAST: the pass may hold fast-mode ops.  Returns x of the tile's index map.
 template <bool SHFL, bool FAST>
-__device__ __forceinline__ void tile_pass_gates(const PassArgs& A, uint64_t base, double* sre, double* sim,
-                                                uint32_t T) {
+__device__ __forceinline__ uint32_t tile_pass_gates(const PassArgs& A, uint64_t base, double* sre, double* sim,
+                                                    uint32_t T) {
+  uint32_t x = 0;
   for (int gi = 0; gi < A.ngates; ++gi) {
     const TileGate& g = A.gates[gi];
     if constexpr (SHFL) {
@@ -509,64 +372,57 @@ __device__ __forceinline__ void tile_pass_gates(const PassArgs& A, uint64_t base
     }
     if ((base & g.g_ones) != g.g_ones || (base & g.g_zeros) != 0) continue;  // uniform per tile
     if (g.cond >= 0 && A.outcomes[g.cond] == 0) continue;                   // classical condition
+    const int mode = g.mode;
+    if (mode == TM_MOVE) {
+      x = move_step(g, x);
+      continue;
+    }
+    int gone = -1;
+    if (mode == TM_DIAG_GLOBAL) {
+      gone = (base & g.g_tbit) ? 1 : 0;
+      if (!gone && g.kind != SPZ_GATE_RZ) continue;  // Z / P act on the 1 half only
+    }
     const uint32_t nw = T >> g.npos;
-    switch (g.mode) {
+    Walk W(g, x, FAST ? fx_base_index(g, base) : 0u);
+    switch (mode) {
       case TM_PAIR:
         switch (g.kind) {
-          case SPZ_GATE_H: tile_pair_any<SPZ_GATE_H, TileGate, TileSwizzle>(g, sre, sim, nw); break;
-          case SPZ_GATE_X: tile_pair_any<SPZ_GATE_X, TileGate, TileSwizzle>(g, sre, sim, nw); break;
-          case SPZ_GATE_Y: tile_pair_any<SPZ_GATE_Y, TileGate, TileSwizzle>(g, sre, sim, nw); break;
-          case SPZ_GATE_RX: tile_pair_any<SPZ_GATE_RX, TileGate, TileSwizzle>(g, sre, sim, nw); break;
-          case SPZ_GATE_RY: tile_pair_any<SPZ_GATE_RY, TileGate, TileSwizzle>(g, sre, sim, nw); break;
-#define SPZ_LAZY(FK)                                                              \
-  case FK:                                                                        \
-    if constexpr (FAST) {                                                         \
-      if (g.pm) tile_fast_phase_pm<FK>(g, A.tables + g.ptab, base, sre, sim, nw); \
-      else tile_pair<FK, 1, TileGate, TileSwizzle>(g, sre, sim, nw);              \
-    }                                                                             \
-    break;
-          SPZ_LAZY(FK_LAZY_H)
-          SPZ_LAZY(FK_LAZY_RX_A)
-          SPZ_LAZY(FK_LAZY_RX_B)
-          SPZ_LAZY(FK_LAZY_RY_A)
-          SPZ_LAZY(FK_LAZY_RY_B)
-#undef SPZ_LAZY
-          default: tile_pair_any<SPZ_GATE_U, TileGate, TileSwizzle>(g, sre, sim, nw); break;
+          case SPZ_GATE_H: tile_pair_op<SPZ_GATE_H>(g, W, sre, sim, nw); break;
+          case SPZ_GATE_X: tile_pair_op<SPZ_GATE_X>(g, W, sre, sim, nw); break;
+          case SPZ_GATE_Y: tile_pair_op<SPZ_GATE_Y>(g, W, sre, sim, nw); break;
+          case SPZ_GATE_RX: tile_pair_op<SPZ_GATE_RX>(g, W, sre, sim, nw); break;
+          case SPZ_GATE_RY: tile_pair_op<SPZ_GATE_RY>(g, W, sre, sim, nw); break;
+          case SPZ_GATE_U: tile_pair_op<SPZ_GATE_U>(g, W, sre, sim, nw); break;
+          default:
+            if constexpr (FAST) tile_lazy_op(g, W, A.tables + g.ptab, sre, sim, nw);
         }
         break;
       case TM_PHASE:
-        if constexpr (FAST) {
-          if (g.npos) tile_phase_pm<1>(g, A.tables + g.ptab, base, sre, sim, nw);
-          else tile_phase_pm<0>(g, A.tables + g.ptab, base, sre, sim, nw);
-        }
+        if constexpr (FAST) tile_phase_op(W, A.tables + g.ptab, sre, sim, nw);
         break;
       case TM_LAZY2:
-        if constexpr (FAST) tile_lazy2_pm(g, A.tables + g.ptab, base, sre, sim, nw);
+        if constexpr (FAST) tile_lazy2_op(g, W, A.tables + g.ptab, sre, sim, nw);
         break;
       case TM_DIAG_LOCAL:
-      case TM_DIAG_GLOBAL: {
-        int gone = -1;
-        if (g.mode == TM_DIAG_GLOBAL) {
-          gone = (base & g.g_tbit) ? 1 : 0;
-          if (!gone && g.kind != SPZ_GATE_RZ) break;  // Z / P act on the 1 half only
-        }
+      case TM_DIAG_GLOBAL:
         switch (g.kind) {
-          case SPZ_GATE_Z: tile_diag_any<SPZ_GATE_Z, TileGate, TileSwizzle>(g, sre, sim, nw, gone); break;
-          case SPZ_GATE_P: tile_diag_any<SPZ_GATE_P, TileGate, TileSwizzle>(g, sre, sim, nw, gone); break;
-          default: tile_diag_any<SPZ_GATE_RZ, TileGate, TileSwizzle>(g, sre, sim, nw, gone); break;
+          case SPZ_GATE_Z: tile_diag_op<SPZ_GATE_Z>(g, W, sre, sim, nw, gone); break;
+          case SPZ_GATE_P: tile_diag_op<SPZ_GATE_P>(g, W, sre, sim, nw, gone); break;
+          default: tile_diag_op<SPZ_GATE_RZ>(g, W, sre, sim, nw, gone); break;
         }
         break;
-      }
       default:  // TM_SWAP
-        tile_swap_any<TileGate, TileSwizzle>(g, sre, sim, nw);
+        tile_swap_op(g, W, sre, sim, nw);
     }
     __syncthreads();
   }
+  return x;
 }
 
 // Every gate of the pass on one tile in fixed point, as tile_pass_gates.
 template <bool SHFL>
-__device__ __forceinline__ void fx_pass_gates(const PassArgs& A, uint64_t base, const FxTile& S, uint32_t T) {
+__device__ __forceinline__ uint32_t fx_pass_gates(const PassArgs& A, uint64_t base, const FxTile& S, uint32_t T) {
+  uint32_t x = 0;
   for (int gi = 0; gi < A.ngates; ++gi) {
     const TileGate& g = A.gates[gi];
     if constexpr (SHFL) {
@@ -588,48 +444,41 @@ __device__ __forceinline__ void fx_pass_gates(const PassArgs& A, uint64_t base, 
     }
     if ((base & g.g_ones) != g.g_ones || (base & g.g_zeros) != 0) continue;
     if (g.cond >= 0 && A.outcomes[g.cond] == 0) continue;
+    if (g.mode == TM_MOVE) {
+      x = move_step(g, x);
+      continue;
+    }
     if (g.mode == TM_DIAG_GLOBAL && g.kind != SPZ_GATE_RZ && !(base & g.g_tbit)) continue;
-    fx_tile_gate(g, A.fxtables, base, S, T);
+    fx_tile_gate(g, A.fxtables, base, x, S, T);
     __syncthreads();
   }
+  return x;
 }
 
 // One tile between global and shared memory: `off` gives the global offset of
-// an even tile offset e (e and e + 1 are consecutive, 16-byte aligned).  In
-// shared memory they share a 16-byte slot too, in reverse order when the
-// swizzle flips the low bits.
+// an even tile offset e (e and e + 1 are consecutive, 16-byte aligned).
 template <class Off>
 __device__ __forceinline__ void load_tile(const PassArgs& A, const Off& off, double* sre, double* sim, uint32_t T) {
   for (uint32_t e2 = threadIdx.x; e2 < T / 2; e2 += blockDim.x) {
     const uint32_t e = 2 * e2;
     const uint64_t gi = off(e);
-    double2 r = *reinterpret_cast<const double2*>(A.re + gi);
-    double2 m = *reinterpret_cast<const double2*>(A.im + gi);
-    const uint32_t p = TileSwizzle::at(e) & ~1u;
-    if (p != e) {
-      r = make_double2(r.y, r.x);
-      m = make_double2(m.y, m.x);
-    }
-    *reinterpret_cast<double2*>(sre + p) = r;
-    *reinterpret_cast<double2*>(sim + p) = m;
+    *reinterpret_cast<double2*>(sre + e) = *reinterpret_cast<const double2*>(A.re + gi);
+    *reinterpret_cast<double2*>(sim + e) = *reinterpret_cast<const double2*>(A.im + gi);
   }
 }
 
+// The amplitudes lie where the pass's moves left them (tile_map.cuh).
 template <class Off>
-__device__ __forceinline__ void store_tile(const PassArgs& A, const Off& off, const double* sre, const double* sim,
-                                           uint32_t T) {
-  for (uint32_t e2 = threadIdx.x; e2 < T / 2; e2 += blockDim.x) {
-    const uint32_t e = 2 * e2;
-    const uint64_t gi = off(e);
-    const uint32_t p = TileSwizzle::at(e) & ~1u;
-    double2 r = *reinterpret_cast<const double2*>(sre + p);
-    double2 m = *reinterpret_cast<const double2*>(sim + p);
-    if (p != e) {
-      r = make_double2(r.y, r.x);
-      m = make_double2(m.y, m.x);
-    }
-    *reinterpret_cast<double2*>(A.re + gi) = r;
-    *reinterpret_cast<double2*>(A.im + gi) = m;
+__device__ __forceinline__ void store_tile(const PassArgs& A, const Off& off, uint32_t x, const double* sre,
+                                           const double* sim, uint32_t T) {
+  const TileGate& end = A.gates[A.ngates];
+  Walk W(end, x);
+  const uint32_t odd = end.tmask;
+  for (uint32_t e2 = threadIdx.x, it = 0; e2 < T / 2; e2 += blockDim.x, ++it) {
+    const uint64_t gi = off(2 * e2);
+    const uint32_t p = W.word(it), q = p ^ odd;
+    *reinterpret_cast<double2*>(A.re + gi) = make_double2(sre[p], sre[q]);
+    *reinterpret_cast<double2*>(A.im + gi) = make_double2(sim[p], sim[q]);
   }
 }
 
@@ -665,32 +514,33 @@ __device__ __forceinline__ void fast_tile(const PassArgs& A, uint64_t base, cons
   if (in_fp64) {
     load_tile(A, off, sre, sim, T);
     __syncthreads();
-    tile_pass_gates<SHFL, true>(A, base, sre, sim, T);
-    store_tile(A, off, sre, sim, T);
+    const uint32_t x = tile_pass_gates<SHFL, true>(A, base, sre, sim, T);
+    store_tile(A, off, x, sre, sim, T);
     return;
   }
   if (!nonzero) return;
-  fx_pass_gates<SHFL>(A, base, S, T);
-  for (uint32_t e2 = threadIdx.x; e2 < T / 2; e2 += blockDim.x) {
-    const uint32_t e = 2 * e2;
-    const uint64_t gi = off(e);
-    const double2 x = fx_to_double(S.load(e)), y = fx_to_double(S.load(e + 1));
+  const uint32_t mx = fx_pass_gates<SHFL>(A, base, S, T);
+  const TileGate& end = A.gates[A.ngates];
+  Walk W(end, mx);
+  const uint32_t odd = end.tmask;
+  for (uint32_t e2 = threadIdx.x, it = 0; e2 < T / 2; e2 += blockDim.x, ++it) {
+    const uint64_t gi = off(2 * e2);
+    const uint32_t p = W.word(it);
+    const double2 x = fx_to_double(S.load(p)), y = fx_to_double(S.load(p ^ odd));
     *reinterpret_cast<double2*>(A.re + gi) = make_double2(x.x, y.x);
     *reinterpret_cast<double2*>(A.im + gi) = make_double2(x.y, y.y);
   }
 }
 
 template <bool SHFL, bool FAST>
-__global__ void __launch_bounds__(kTileThreads, FAST ? SPZ_FAST_MIN_BLOCKS : SHFL ? 12 : SPZ_TILE_MIN_BLOCKS)
-    tile_kernel(PassArgs A) {
+__global__ void __maxnreg__(FAST ? SPZ_FAST_REGS : SPZ_TILE_REGS) tile_kernel(PassArgs A) {
   extern __shared__ double smem[];
   const int K = A.k;
   const uint32_t T = 1u << K;
   double* sre = smem;
   double* sim = smem + T;
   // Row offsets >> c (their bits are local qubits >= c, so 32 bits hold them
-  // for up to 34 qubits): half the shared memory of 64-bit entries, which
-  // lets a 13th block of 2^10-amplitude tiles onto an SM.
+  // for up to 34 qubits): half the shared memory of 64-bit entries.
   uint32_t* rowoff = reinterpret_cast<uint32_t*>(smem + 2 * T);
   const uint32_t nrows = 1u << A.nhigh;
   int32_t* sexp = reinterpret_cast<int32_t*>(rowoff + (nrows + 1u & ~1u));  // FAST: the amplitudes' exponents
@@ -716,8 +566,8 @@ __global__ void __launch_bounds__(kTileThreads, FAST ? SPZ_FAST_MIN_BLOCKS : SHF
     } else {
       load_tile(A, off, sre, sim, T);
       __syncthreads();
-      tile_pass_gates<SHFL, false>(A, base, sre, sim, T);
-      store_tile(A, off, sre, sim, T);
+      const uint32_t x = tile_pass_gates<SHFL, false>(A, base, sre, sim, T);
+      store_tile(A, off, x, sre, sim, T);
     }
     __syncthreads();
   }
@@ -852,8 +702,8 @@ __global__ void __launch_bounds__(kTileThreads) tile_kernel_tma(PassArgs A, cons
     if constexpr (FAST) {
       fast_tile<false>(A, base, off, true, sre, sim, reinterpret_cast<int32_t*>(rowoff + nrows), T);
     } else {
-      tile_pass_gates<false, false>(A, base, sre, sim, T);
-      store_tile(A, off, sre, sim, T);
+      const uint32_t x = tile_pass_gates<false, false>(A, base, sre, sim, T);
+      store_tile(A, off, x, sre, sim, T);
     }
     __syncthreads();
     if (!PREFETCH && next < A.ntiles) issue(next, 0);
@@ -1028,6 +878,13 @@ FlatTables flatten(const std::vector<GateApp>& gates, const std::vector<PhaseTab
   return f;
 }
 
+DiagCoef diag_coef(double re1, double im1) {
+  uint64_t rb, ib;
+  std::memcpy(&rb, &re1, sizeof rb);
+  std::memcpy(&ib, &im1, sizeof ib);
+  return diag_prepare(re1, im1, rb, ib);
+}
+
 // Build the device description of a gate inside a pass with local qubits `L`.
 TileGate tile_gate(const GateApp& g, const std::vector<int>& local, const std::vector<PhaseTable>* tables = nullptr,
                    const std::vector<uint32_t>* table_offsets = nullptr) {
@@ -1038,6 +895,8 @@ TileGate tile_gate(const GateApp& g, const std::vector<int>& local, const std::v
   t.kind = g.kind;
   t.c = g.c;
   t.cond = g.cond;
+  if (g.kind == SPZ_GATE_P) t.d = diag_coef(g.c.cs, g.c.sn);
+  if (g.kind == SPZ_GATE_RZ) t.d = diag_coef(g.c.d1re, g.c.d1im);
   if (g.kind >= FK_LAZY_H && g.kind <= FK_LAZY_RY_B) {
     const FxLazy x = fx_lazy(g.kind, g.c.cs);
     t.fx1 = fx_coef(std::isfinite(x.t) ? x.t : 0.0);
@@ -1348,10 +1207,32 @@ uint64_t op_fp64_ops(uint32_t n, const GateApp& g, const std::vector<PhaseTable>
   return gate_fp64_ops(n, g);
 }
 
-// Resident blocks per SM for a tile pass of `threads` x `smem` and the SM
-// count; the grid of a tile pass is one wave of them (each block loops over
-// tiles), so no block waits for a second wave.  Cached per device and tile
-// size (kernel attributes are per device); callers may be on several threads.
+// The SM count of a device; callers may be on several threads.
+int device_sms(int device, int* out) {
+  static std::mutex mu;
+  static int sms[kMaxDevices] = {};
+  if (device < 0 || device >= kMaxDevices) return fail(SPZ_ERR_INVALID_ARGUMENT, "device index out of range");
+  std::lock_guard<std::mutex> lock(mu);
+  if (!sms[device]) SPZ_CUDA(cudaDeviceGetAttribute(&sms[device], cudaDevAttrMultiProcessorCount, device));
+  *out = sms[device];
+  return SPZ_OK;
+}
+
+// Threads of a tile pass's blocks.  Many tiles: kTileThreads (many small blocks
+// keep the FP64 pipe busy through the barriers).  With fewer tiles than fill
+// the SMs, every op is a chain of latencies, which more threads per tile
+// shorten: doubled until the GPU has kTileSmThreads threads per SM, at most
+// one thread per pair.  Measured, exact QFT: 16 qubits 260 us with 128 threads,
+// 230 with 256; 18 qubits 328 and 287; 20 qubits (1024 tiles) 653 with 64, 814
+// with 128; 512 threads no faster.  (`may_grow`: warp-shuffle runs and TMA staging keep
+// kTileThreads.)
+int tile_threads(uint32_t T, uint64_t ntiles, int sms, bool may_grow) {
+  int t = (int)std::min<uint32_t>(kTileThreads, std::max<uint32_t>(32, T / 2));
+  while (may_grow && t < kTileMaxThreads && (uint32_t)t < T / 2 && ntiles * (uint64_t)t < (uint64_t)sms * kTileSmThreads)
+    t *= 2;
+  return t;
+}
+
 using TileKernel = void (*)(PassArgs);
 TileKernel tile_kernel_for(bool shfl, bool fast) {
   if (fast) return shfl ? tile_kernel<true, true> : tile_kernel<false, true>;
@@ -1365,16 +1246,19 @@ size_t tile_smem(int k, int nhigh, bool fast) {
   return 2 * T * sizeof(double) + ((rows + 1) & ~(size_t)1) * sizeof(uint32_t) + (fast ? T * sizeof(int32_t) : 0);
 }
 
+// Resident blocks per SM for a tile pass of `threads` x `smem` and the SM
+// count; the grid of a tile pass is one wave of them (each block loops over
+// tiles), so no block waits for a second wave.  Cached per device and tile
+// size (kernel attributes are per device); callers may be on several threads.
 int tile_launch_shape(int device, int threads, size_t smem, int* resident_out, int* sms_out, bool shfl, bool fast) {
   static std::mutex mu;
-  static int sms[kMaxDevices] = {};
-  // by log2 of the tile, 32 / 64 threads, and the instantiation
-  static int resident[kMaxDevices][kTileMaxK + 2][2][4] = {};
-  if (device < 0 || device >= kMaxDevices) return fail(SPZ_ERR_INVALID_ARGUMENT, "device index out of range");
+  static bool ready[kMaxDevices] = {};
+  // by log2 of the tile, log2 of the threads (from 32), and the instantiation
+  static int resident[kMaxDevices][kTileMaxK + 2][6][4] = {};
+  int sms = 0;
+  if (int rc = device_sms(device, &sms)) return rc;
   std::lock_guard<std::mutex> lock(mu);
-  if (!sms[device]) {
-    int count = 0;
-    SPZ_CUDA(cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, device));
+  if (!ready[device]) {
     for (int v = 0; v < 4; ++v) {
       const void* fn = (const void*)tile_kernel_for(v & 1, v & 2);
       const int max_smem = (int)tile_smem(kTileMaxK, kTileMaxK - kTileLowBits, v & 2);
@@ -1382,11 +1266,11 @@ int tile_launch_shape(int device, int threads, size_t smem, int* resident_out, i
       SPZ_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout,
                                     cudaSharedmemCarveoutMaxShared));
     }
-    sms[device] = count;
+    ready[device] = true;
   }
   int lg = 0;  // the largest lg with 2 x 8 B x 2^lg <= smem (the tile's re and im)
   while (lg <= kTileMaxK && (16ull << (lg + 1)) <= smem) ++lg;
-  int& r = resident[device][lg][threads > 32 ? 1 : 0][(shfl ? 1 : 0) + (fast ? 2 : 0)];
+  int& r = resident[device][lg][31 - __builtin_clz((unsigned)threads) - 5][(shfl ? 1 : 0) + (fast ? 2 : 0)];
   if (!r) {
     int per_sm = 0;
     const void* fn = (const void*)tile_kernel_for(shfl, fast);
@@ -1394,7 +1278,7 @@ int tile_launch_shape(int device, int threads, size_t smem, int* resident_out, i
     r = std::max(1, per_sm);
   }
   *resident_out = r;
-  *sms_out = sms[device];
+  *sms_out = sms;
   return SPZ_OK;
 }
 
@@ -1632,9 +1516,12 @@ int run_gates_io(spz_state_t h, const std::vector<GateApp>& gates_in, uint32_t f
         const size_t r = mark_shuffle_runs(pg.data(), pg.size(), (int)P.local.size());
         if (st) st->shuffle_gates += r;
       }
+      map_pass(&pg, (int)P.local.size(), (flags & SPZ_EXEC_SHUFFLE) != 0);
+      counts.push_back(pg.size() - 1);  // the last one is the store's walk
       all.insert(all.end(), pg.begin(), pg.end());
+    } else {
+      counts.push_back(0);
     }
-    counts.push_back(pg.size());
   }
   TileGate* dgates = nullptr;
   const double2* dtables = nullptr;
@@ -1662,14 +1549,12 @@ int run_gates_io(spz_state_t h, const std::vector<GateApp>& gates_in, uint32_t f
   // is cleared here and read back at the end of the run.
   const bool shfl = (flags & SPZ_EXEC_SHUFFLE) != 0;
   bool use_tma = false;
-#if !SPZ_TILE_SWIZZLE
   if ((flags & (SPZ_EXEC_TMA | SPZ_EXEC_TMA_PREFETCH)) && n >= 5) {
     int rc = ensure_tma_maps(h);
     if (rc) return rc;
     SPZ_CUDA(cudaMemsetAsync(h->tma_err, 0, sizeof(int), h->stream));
     use_tma = true;
   }
-#endif
   auto pass_slab_q = [&](const PlannedPass& P) -> int {
     if (!io || n < 3 || !tiled(P) || (n - P.local.size()) < 3) return -1;
     uint64_t local_mask = 0;
@@ -1718,10 +1603,11 @@ int run_gates_io(spz_state_t h, const std::vector<GateApp>& gates_in, uint32_t f
     A.ngates = (int)counts[p];
     const uint32_t T = 1u << A.k;
     const size_t smem = tile_smem(A.k, A.nhigh, fast);
-    const int threads = h->tile_threads ? h->tile_threads
-                                        : (int)std::min<uint32_t>(kTileThreads, std::max<uint32_t>(32, T / 2));
     int resident = 0, sms = 0;
-    int rc = tile_launch_shape(h->device, threads, smem, &resident, &sms, shfl, fast);
+    int rc = device_sms(h->device, &sms);
+    if (rc) return rc;
+    const int threads = h->tile_threads ? h->tile_threads : tile_threads(T, ntiles, sms, !shfl && !use_tma);
+    rc = tile_launch_shape(h->device, threads, smem, &resident, &sms, shfl, fast);
     if (rc) return rc;
     if (use_tma && !A.slab_on && A.c == kTileLowBits && A.k >= kTileLowBits + 2) {
       const bool pre = (flags & SPZ_EXEC_TMA_PREFETCH) != 0;
@@ -2270,9 +2156,12 @@ int build_program(spz_program_t p, const spz_op* ops, size_t nops, uint32_t flag
       if (fast) p->stats.fp64_ops -= fuse_lazy_pairs(pg, P.gates, tables, &flat, n);
       if (flags & SPZ_EXEC_SHUFFLE)
         p->stats.shuffle_gates += mark_shuffle_runs(pg.data(), pg.size(), (int)P.local.size());
+      map_pass(&pg, (int)P.local.size(), (flags & SPZ_EXEC_SHUFFLE) != 0);
+      counts.push_back(pg.size() - 1);  // the last one is the store's walk
       all.insert(all.end(), pg.begin(), pg.end());
+    } else {
+      counts.push_back(0);
     }
-    counts.push_back(pg.size());
   }
   const size_t gbytes = (all.size() * sizeof(TileGate) + 255) / 256 * 256;
   const size_t tbytes = flat.entries.size() * sizeof(double2);
@@ -2309,11 +2198,13 @@ int build_program(spz_program_t p, const spz_op* ops, size_t nops, uint32_t flag
     A.ngates = (int)counts[q];
     const uint32_t T = 1u << A.k;
     pp.smem = tile_smem(A.k, A.nhigh, fast);
-    pp.threads = (int)std::min<uint32_t>(kTileThreads, std::max<uint32_t>(32, T / 2));
+    int resident = 0, sms = 0;
+    int rc = device_sms(p->device, &sms);
+    if (rc) return rc;
+    pp.threads = tile_threads(T, A.ntiles, sms, !(flags & SPZ_EXEC_SHUFFLE));
     pp.shfl = (flags & SPZ_EXEC_SHUFFLE) != 0;
     pp.fast = fast;
-    int resident = 0, sms = 0;
-    int rc = tile_launch_shape(p->device, pp.threads, pp.smem, &resident, &sms, pp.shfl, pp.fast);
+    rc = tile_launch_shape(p->device, pp.threads, pp.smem, &resident, &sms, pp.shfl, pp.fast);
     if (rc) return rc;
     pp.blocks = std::min<uint64_t>(A.ntiles, (uint64_t)sms * resident);
     p->stats.tile_passes++;

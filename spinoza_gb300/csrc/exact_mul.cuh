@@ -69,6 +69,23 @@ SPZ_HD MulCoef mul_prepare(uint64_t c, MulRange& r) {
   return m;
 }
 
+// The diagonal entry (re1, im1) of P on its 1 half, or of RZ on 1, prepared.
+struct alignas(16) DiagCoef {
+  MulRange range;
+  MulCoef mre, mim;
+  double re1, im1;
+};
+
+SPZ_HD DiagCoef diag_prepare(double re1, double im1, uint64_t re1_bits, uint64_t im1_bits) {
+  DiagCoef d;
+  d.range = mul_range_all();
+  d.mre = mul_prepare(re1_bits, d.range);
+  d.mim = mul_prepare(im1_bits, d.range);
+  d.re1 = re1;
+  d.im1 = im1;
+  return d;
+}
+
 SPZ_HD bool mul_ok(uint64_t y, const MulRange& r) {
   return (((uint32_t)(y >> 32) & 0x7FFFFFFFu) - r.lo) < r.span;
 }

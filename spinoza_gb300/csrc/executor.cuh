@@ -5,6 +5,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "exact_mul.cuh"
 #include "fixed_point.cuh"
 
 namespace spz {
@@ -18,22 +19,35 @@ constexpr int kTileLowBits = 3;   // qubits 0..2 always local: 64-byte contiguou
 // the FP64 pipe stays busier with many independent small blocks per SM than
 // with a few large ones.  Measured on the 30-qubit brickwork, fast mode, share
 // of the DFMA issue rate: 2^12 tiles x 256 threads x 3 blocks 0.81; 2^11 x 128
-// x 6 0.84; 2^10 x 64 x 12 0.86 (exact mode 0.86-0.87 for all three).  With
-// 32-bit row offsets a block needs 16.5 KiB (+1 KiB the runtime reserves), so
-// 13 fit an SM's 228 KiB; 13 against 12 measured the same on the 30-qubit
-// brickwork (fast 4,472 / 4,476 ms, exact 8,360 / 8,355 ms per step).
+// x 6 0.84; 2^10 x 64 x 12 0.86 (exact mode 0.86-0.87 for all three).
 #ifndef SPZ_TILE_THREADS
 #define SPZ_TILE_THREADS 64
 #endif
-#ifndef SPZ_TILE_MIN_BLOCKS
-#define SPZ_TILE_MIN_BLOCKS 13  // 13 x (16 KiB tile + 0.5 KiB row table + 1 KiB reserved) <= 228 KiB
+// A state of few tiles gets blocks of up to kTileMaxThreads, so that every SM
+// still has about kTileSmThreads threads to hide latencies with (tile_threads
+// in circuit.cu).
+#ifndef SPZ_TILE_MAX_THREADS
+#define SPZ_TILE_MAX_THREADS 256
 #endif
-#ifndef SPZ_FAST_MIN_BLOCKS
-#define SPZ_FAST_MIN_BLOCKS 10  // fast mode: 4 KiB of exponents more per tile
+constexpr int kTileMaxThreads = SPZ_TILE_MAX_THREADS;
+constexpr int kTileSmThreads = 400;
+// Registers a thread: 12 blocks of 64 threads on an SM in the exact mode (26
+// qubits, 10 brickwork layers: 171.1 ms; 72 registers and 13 blocks 177.7), 10
+// in the fast mode, whose tiles take 21 KiB.
+#ifndef SPZ_TILE_REGS
+#define SPZ_TILE_REGS 80
+#endif
+#ifndef SPZ_FAST_REGS
+#define SPZ_FAST_REGS 96
 #endif
 constexpr int kTileThreads = SPZ_TILE_THREADS;
 
-enum TileMode { TM_PAIR = 0, TM_DIAG_LOCAL = 1, TM_DIAG_GLOBAL = 2, TM_SWAP = 3, TM_PHASE = 4, TM_LAZY2 = 5 };
+// TM_MOVE: X, CX or SWAP as a step of the tile's index map; TM_END: the walk of
+// the tile's store (tile_map.cuh).
+enum TileMode {
+  TM_PAIR = 0, TM_DIAG_LOCAL = 1, TM_DIAG_GLOBAL = 2, TM_SWAP = 3, TM_PHASE = 4, TM_LAZY2 = 5, TM_MOVE = 6, TM_END = 7
+};
+enum MoveKind { MV_X = 0, MV_CX1 = 1, MV_CX0 = 2, MV_SWAP = 3 };
 
 struct TileGate {
   int32_t kind;
@@ -76,6 +90,16 @@ struct TileGate {
   FxCoef fx1, fx2;
   uint32_t fxswaps, fxturns;
   int32_t fexp;
+  // The op's walk (circuit executor, tile_map.cuh): word(m) = wk0 ^ XOR of
+  // wcol[i] over the bits i of item m ^ XOR of wx[q] over the bits q of the
+  // tile's x; bits 0-15 the item's slot, 16 and up its phase index (or, for a
+  // TM_DIAG_LOCAL, its target bit).  tmask, tmask2: what flips tbit, tbit2.
+  // TM_MOVE: tmask, tmask2 are the bit numbers of target and control.
+  alignas(16) uint32_t wk0;
+  uint32_t tmask, tmask2, wpad;
+  uint32_t wcol[12];  // kTileMaxK used: read as three 16-byte words
+  uint32_t wx[kTileMaxK];
+  DiagCoef d;  // P, RZ: the coefficients prepared for DiagGate
 };
 
 // The descriptor of gate g inside a tile pass whose local qubits are `local`

@@ -157,22 +157,12 @@ struct PairGate {
 // Diagonal gates on one amplitude; `one` is the amplitude's target bit.  RZ's
 // entries are (re, im) = (cos, -sin) on 0 and (cos, sin) on 1.
 template <int KIND>
-struct DiagGate {
-  MulRange range = mul_range_all();
-  MulCoef mre{}, mim{};
-  double re1 = 0.0, im1 = 0.0;  // the entry on 1
-
-  __device__ __forceinline__ explicit DiagGate(const Coef& c) {
-    if constexpr (KIND == SPZ_GATE_P) {
-      re1 = c.cs;
-      im1 = c.sn;
-    } else if constexpr (KIND == SPZ_GATE_RZ) {
-      re1 = c.d1re;
-      im1 = c.d1im;
-    }
+struct DiagGate : DiagCoef {
+  __device__ __forceinline__ explicit DiagGate(const DiagCoef& d) : DiagCoef(d) {}
+  __device__ __forceinline__ explicit DiagGate(const Coef& c) : DiagCoef{} {
     if constexpr (KIND != SPZ_GATE_Z) {
-      mre = mul_prepare(dbits(re1), range);
-      mim = mul_prepare(dbits(im1), range);
+      const double r = KIND == SPZ_GATE_P ? c.cs : c.d1re, i = KIND == SPZ_GATE_P ? c.sn : c.d1im;
+      *static_cast<DiagCoef*>(this) = diag_prepare(r, i, dbits(r), dbits(i));
     }
   }
 

@@ -11,7 +11,7 @@
 #include "executor.cuh"
 #include "fixed_point.cuh"
 #include "gate_math.cuh"
-#include "tile_ops.cuh"
+#include "tile_map.cuh"
 
 namespace spz {
 
@@ -75,36 +75,34 @@ __device__ __forceinline__ void fx_phase(FxAmp& a, const int4& w, int32_t fexp) 
   fx_settle<1>(&a, a.e + fexp);
 }
 
-static __device__ void fx_tile_lazy(const TileGate& g, const int4* __restrict__ tables, uint64_t base,
+static __device__ void fx_tile_lazy(const TileGate& g, const int4* __restrict__ tables, Walk W,
                                     const FxTile& S, uint32_t npairs) {
-  const Enumerator<1, TileGate> E(g);
-  const uint32_t tbit = g.tbit, bidx = fx_base_index(g, base), swaps = g.fxswaps, turns = g.fxturns;
+  const uint32_t tmask = g.tmask, swaps = g.fxswaps, turns = g.fxturns;
   const bool has_w = g.pm > 0;
   const int4* tab = tables + g.ptab;
   const FxCoef t = g.fx1;
-  for (uint32_t m = threadIdx.x; m < npairs; m += blockDim.x) {
-    const uint32_t s0 = E(m), s1 = s0 | tbit;
+  for (uint32_t m = threadIdx.x, it = 0; m < npairs; m += blockDim.x, ++it) {
+    const uint32_t word = W.word(it), s0 = word & 0xFFFFu, s1 = s0 ^ tmask;
     FxAmp a[2] = {S.load(s0), S.load(s1)};
     int4 w = make_int4(0, 0, 0, 0);
-    if (has_w) w = __ldg(tab + fx_index(g, bidx, s0));
+    if (has_w) w = __ldg(tab + (word >> 16));
     fx_lazy_pair(a, t, has_w, w, swaps, turns);
     S.store(s0, a[0]);
     S.store(s1, a[1]);
   }
 }
 
-// Two lazy rotations on blocks of four amplitudes, as tile_lazy2 (circuit.cu):
+// Two lazy rotations on blocks of four amplitudes, as tile_lazy2_op (circuit.cu):
 // three phases, the first rotation along b1, the second along b2.
-static __device__ void fx_tile_lazy2(const TileGate& g, const int4* __restrict__ tables, uint64_t base,
+static __device__ void fx_tile_lazy2(const TileGate& g, const int4* __restrict__ tables, Walk W,
                                      const FxTile& S, uint32_t nblocks) {
-  const Enumerator<2, TileGate> E(g);
-  const uint32_t b1 = g.tbit, b2 = g.tbit2, bidx = fx_base_index(g, base), swaps = g.fxswaps, turns = g.fxturns;
+  const uint32_t b1 = g.tmask, b2 = g.tmask2, swaps = g.fxswaps, turns = g.fxturns;
   const int4* tab = tables + g.ptab;
   const FxCoef t1 = g.fx1, t2 = g.fx2;
-  for (uint32_t m = threadIdx.x; m < nblocks; m += blockDim.x) {
-    const uint32_t e = E(m);
-    const int4* row = tab + 3 * fx_index(g, bidx, e);
-    FxAmp a[4] = {S.load(e), S.load(e | b1), S.load(e | b2), S.load(e | b1 | b2)};
+  for (uint32_t m = threadIdx.x, it = 0; m < nblocks; m += blockDim.x, ++it) {
+    const uint32_t word = W.word(it), e = word & 0xFFFFu;
+    const int4* row = tab + 3 * (word >> 16);
+    FxAmp a[4] = {S.load(e), S.load(e ^ b1), S.load(e ^ b2), S.load(e ^ b1 ^ b2)};
     const int32_t X = fx_align<4>(a);
 #pragma unroll
     for (int j = 1; j < 4; ++j) {
@@ -129,21 +127,20 @@ static __device__ void fx_tile_lazy2(const TileGate& g, const int4* __restrict__
     }
     fx_settle<4>(a, X);
     S.store(e, a[0]);
-    S.store(e | b1, a[1]);
-    S.store(e | b2, a[2]);
-    S.store(e | b1 | b2, a[3]);
+    S.store(e ^ b1, a[1]);
+    S.store(e ^ b2, a[2]);
+    S.store(e ^ b1 ^ b2, a[3]);
   }
 }
 
-static __device__ void fx_tile_phase(const TileGate& g, const int4* __restrict__ tables, uint64_t base,
+static __device__ void fx_tile_phase(const TileGate& g, const int4* __restrict__ tables, Walk W,
                                      const FxTile& S, uint32_t nelem) {
-  const Enumerator<-1, TileGate> E(g);
-  const uint32_t bidx = fx_base_index(g, base);
   const int4* tab = tables + g.ptab;
-  for (uint32_t m = threadIdx.x; m < nelem; m += blockDim.x) {
-    const uint32_t e = E(m);
+  const int32_t fexp = g.fexp;
+  for (uint32_t m = threadIdx.x, it = 0; m < nelem; m += blockDim.x, ++it) {
+    const uint32_t word = W.word(it), e = word & 0xFFFFu;
     FxAmp a = S.load(e);
-    fx_phase(a, __ldg(tab + fx_index(g, bidx, e)), g.fexp);
+    fx_phase(a, __ldg(tab + (word >> 16)), fexp);
     S.store(e, a);
   }
 }
@@ -177,42 +174,43 @@ __device__ __forceinline__ void fx_exact_diag(const TileGate& g, bool one, FxAmp
   }
   if (!one && g.kind == SPZ_GATE_P) return;
   double2 x = fx_to_double(a);
-  if (g.kind == SPZ_GATE_P) DiagGate<SPZ_GATE_P>(g.c)(one, x.x, x.y);
-  else DiagGate<SPZ_GATE_RZ>(g.c)(one, x.x, x.y);
+  if (g.kind == SPZ_GATE_P) DiagGate<SPZ_GATE_P>(g.d)(one, x.x, x.y);
+  else DiagGate<SPZ_GATE_RZ>(g.d)(one, x.x, x.y);
   a = fx_from_double(x.x, x.y);
 }
 
-static __device__ void fx_tile_exact(const TileGate& g, uint64_t base, const FxTile& S, uint32_t nw) {
-  const Enumerator<-1, TileGate> E(g);
-  const uint32_t tbit = g.tbit, tbit2 = g.tbit2;
+static __device__ void fx_tile_exact(const TileGate& g, uint64_t base, Walk W, const FxTile& S, uint32_t nw) {
+  const uint32_t tmask = g.tmask, tmask2 = g.tmask2;
   const int mode = g.mode;
   const bool gone = mode == TM_DIAG_GLOBAL && (base & g.g_tbit) != 0;
-  for (uint32_t m = threadIdx.x; m < nw; m += blockDim.x) {
-    const uint32_t e = E(m);
+  for (uint32_t m = threadIdx.x, it = 0; m < nw; m += blockDim.x, ++it) {
+    const uint32_t word = W.word(it), e = word & 0xFFFFu;
     if (mode == TM_SWAP) {
-      const FxAmp a = S.load(e | tbit2), b = S.load(e | tbit);
-      S.store(e | tbit2, b);
-      S.store(e | tbit, a);
+      const FxAmp a = S.load(e ^ tmask2), b = S.load(e ^ tmask);
+      S.store(e ^ tmask2, b);
+      S.store(e ^ tmask, a);
     } else if (mode == TM_PAIR) {
-      FxAmp a = S.load(e), b = S.load(e | tbit);
+      FxAmp a = S.load(e), b = S.load(e ^ tmask);
       fx_exact_pair(g, a, b);
       S.store(e, a);
-      S.store(e | tbit, b);
+      S.store(e ^ tmask, b);
     } else {
       FxAmp a = S.load(e);
-      fx_exact_diag(g, mode == TM_DIAG_GLOBAL ? gone : (e & tbit) != 0, a);
+      fx_exact_diag(g, mode == TM_DIAG_GLOBAL ? gone : (word >> 16) != 0, a);
       S.store(e, a);
     }
   }
 }
 
+// Op g on the tile; x: the tile's (tile_map.cuh).
 static __device__ __forceinline__ void fx_tile_gate(const TileGate& g, const int4* __restrict__ tables, uint64_t base,
-                                                    const FxTile& S, uint32_t T) {
+                                                    uint32_t x, const FxTile& S, uint32_t T) {
   const uint32_t nw = T >> g.npos;
-  if (g.mode == TM_LAZY2) fx_tile_lazy2(g, tables, base, S, nw);
-  else if (g.mode == TM_PHASE) fx_tile_phase(g, tables, base, S, nw);
-  else if (g.mode == TM_PAIR && g.kind >= FK_LAZY_H) fx_tile_lazy(g, tables, base, S, nw);
-  else fx_tile_exact(g, base, S, nw);
+  Walk W(g, x, fx_base_index(g, base));
+  if (g.mode == TM_LAZY2) fx_tile_lazy2(g, tables, W, S, nw);
+  else if (g.mode == TM_PHASE) fx_tile_phase(g, tables, W, S, nw);
+  else if (g.mode == TM_PAIR && g.kind >= FK_LAZY_H) fx_tile_lazy(g, tables, W, S, nw);
+  else fx_tile_exact(g, base, W, S, nw);
 }
 
 // A run of gates inside rows of 32 amplitudes (SPZ_EXEC_SHUFFLE, see

@@ -1,6 +1,5 @@
-// Gate ops on a tile of amplitudes held in shared memory, shared by the fused
-// circuit executor (circuit.cu) and the batched engine (batch.cu).  A gate
-// descriptor G provides: pos[] / npos (sorted tile-offset bits inserted as
+// Gate ops on a tile of amplitudes held in shared memory, for the batched engine
+// (batch.cu) and the fused adjoint sweep (adjoint.cu).  A gate descriptor G provides: pos[] / npos (sorted tile-offset bits inserted as
 // zeros by the enumeration: target and local controls), l_ones (local bits
 // set: controls, and the target of a diagonal gate that acts on its 1 half),
 // tbit / tbit2 (the target's tile bit; SWAP's second), and the gate's Coef c.
@@ -49,26 +48,6 @@ struct Enumerator<-1, G> {
   }
 };
 
-// Shared-memory layout of a tile: amplitude e lives at SW::at(e).
-// NoSwizzle keeps e.  NibbleSwizzle flips the low four bits of e when bit 4
-// is set: the 16 lanes of a half-warp that read s0 (or s1) of a pair op with
-// its target at tile bit 0-3 then hit 16 distinct 8-byte bank slots instead
-// of 8 twice (a 2-way conflict); accesses whose low four bits run through all
-// values in a half-warp are unaffected.  An involution.
-struct NoSwizzle {
-  __device__ __forceinline__ static uint32_t at(uint32_t e) { return e; }
-};
-struct NibbleSwizzle {
-  __device__ __forceinline__ static uint32_t at(uint32_t e) { return e ^ ((0u - ((e >> 4) & 1u)) & 15u); }
-};
-
-// Unroll factor of the per-pair loops (independent iterations in flight per
-// thread); 2 measured no faster than 1 on the 30-qubit brickwork.
-#ifndef SPZ_TILE_UNROLL
-#define SPZ_TILE_UNROLL 1
-#endif
-constexpr int kTileUnroll = SPZ_TILE_UNROLL;
-
 // Dispatch on the op's insertion count: 0-3 specialised, more generic.
 #define SPZ_BY_NPOS(npos, CALL) \
   switch (npos) {               \
@@ -79,102 +58,63 @@ constexpr int kTileUnroll = SPZ_TILE_UNROLL;
     default: CALL(-1); break;   \
   }
 
-// Pairs handled per loop iteration and thread.  The pairs of one op are
-// disjoint, but the compiler cannot prove that the next pair's shared-memory
-// loads do not alias this pair's stores, so unrolling alone cannot overlap
-// them; the batched loop loads kTileBatch pairs, computes them, then stores.
-// Measured on the 30-qubit brickwork with 2: fast mode 4% slower (80
-// registers instead of 72), exact mode 0.7% faster; 4 spills.  So 1.
-#ifndef SPZ_TILE_BATCH
-#define SPZ_TILE_BATCH 1
-#endif
-constexpr int kTileBatch = SPZ_TILE_BATCH;
-
-template <int KIND, int NPOS, class G, class SW = NoSwizzle>
+template <int KIND, int NPOS, class G>
 __device__ __forceinline__ void tile_pair(const G& g, double* sre, double* sim, uint32_t npairs) {
   const Enumerator<NPOS, G> E(g);
   const uint32_t tbit = g.tbit;
   const PairGate<KIND> op(g.c);
-  if constexpr (kTileBatch > 1) {
-    const uint32_t step = blockDim.x;
-    for (uint32_t m0 = threadIdx.x; m0 < npairs; m0 += kTileBatch * step) {
-      uint32_t s0[kTileBatch], s1[kTileBatch];
-      double a[kTileBatch], b[kTileBatch], x[kTileBatch], d[kTileBatch];
-#pragma unroll
-      for (int u = 0; u < kTileBatch; ++u) {
-        const uint32_t m = m0 + u * step;
-        const uint32_t e0 = E(m < npairs ? m : m0);
-        s0[u] = SW::at(e0);
-        s1[u] = SW::at(e0 | tbit);
-        a[u] = sre[s0[u]]; b[u] = sim[s0[u]]; x[u] = sre[s1[u]]; d[u] = sim[s1[u]];
-      }
-#pragma unroll
-      for (int u = 0; u < kTileBatch; ++u) op(a[u], b[u], x[u], d[u]);
-#pragma unroll
-      for (int u = 0; u < kTileBatch; ++u) {
-        if (m0 + u * step < npairs) {
-          sre[s0[u]] = a[u]; sim[s0[u]] = b[u]; sre[s1[u]] = x[u]; sim[s1[u]] = d[u];
-        }
-      }
-    }
-  } else {
-#pragma unroll kTileUnroll
-    for (uint32_t m = threadIdx.x; m < npairs; m += blockDim.x) {
-      const uint32_t e0 = E(m);
-      const uint32_t s0 = SW::at(e0), s1 = SW::at(e0 | tbit);
-      double a = sre[s0], b = sim[s0], x = sre[s1], d = sim[s1];
-      op(a, b, x, d);
-      sre[s0] = a; sim[s0] = b; sre[s1] = x; sim[s1] = d;
-    }
+  for (uint32_t m = threadIdx.x; m < npairs; m += blockDim.x) {
+    const uint32_t s0 = E(m), s1 = s0 | tbit;
+    double a = sre[s0], b = sim[s0], x = sre[s1], d = sim[s1];
+    op(a, b, x, d);
+    sre[s0] = a; sim[s0] = b; sre[s1] = x; sim[s1] = d;
   }
 }
 
-template <int KIND, class G, class SW = NoSwizzle>
+template <int KIND, class G>
 __device__ __forceinline__ void tile_pair_any(const G& g, double* sre, double* sim, uint32_t npairs) {
-#define SPZ_CALL(N) tile_pair<KIND, N, G, SW>(g, sre, sim, npairs)
+#define SPZ_CALL(N) tile_pair<KIND, N, G>(g, sre, sim, npairs)
   SPZ_BY_NPOS(g.npos, SPZ_CALL)
 #undef SPZ_CALL
 }
 
-template <int KIND, int NPOS, class G, class SW = NoSwizzle>
+template <int KIND, int NPOS, class G>
 __device__ __forceinline__ void tile_diag(const G& g, double* sre, double* sim, uint32_t nelem, int global_one) {
   const Enumerator<NPOS, G> E(g);
   const uint32_t tbit = g.tbit;
   const DiagGate<KIND> op(g.c);
   for (uint32_t m = threadIdx.x; m < nelem; m += blockDim.x) {
-    const uint32_t e0 = E(m);
-    const bool one = global_one >= 0 ? global_one != 0 : (e0 & tbit) != 0;
-    const uint32_t e = SW::at(e0);
+    const uint32_t e = E(m);
     double r = sre[e], i = sim[e];
-    op(one, r, i);
+    op(global_one >= 0 ? global_one != 0 : (e & tbit) != 0, r, i);
     sre[e] = r; sim[e] = i;
   }
 }
 
-template <int KIND, class G, class SW = NoSwizzle>
+template <int KIND, class G>
 __device__ __forceinline__ void tile_diag_any(const G& g, double* sre, double* sim, uint32_t nelem,
                                               int global_one) {
-#define SPZ_CALL(N) tile_diag<KIND, N, G, SW>(g, sre, sim, nelem, global_one)
+#define SPZ_CALL(N) tile_diag<KIND, N, G>(g, sre, sim, nelem, global_one)
   SPZ_BY_NPOS(g.npos, SPZ_CALL)
 #undef SPZ_CALL
 }
 
-template <int NPOS, class G, class SW = NoSwizzle>
+template <int NPOS, class G>
 __device__ __forceinline__ void tile_swap(const G& g, double* sre, double* sim, uint32_t nw) {
   const Enumerator<NPOS, G> E(g);
   const uint32_t t1 = g.tbit, t2 = g.tbit2;
   for (uint32_t m = threadIdx.x; m < nw; m += blockDim.x) {
     const uint32_t b0 = E(m);
-    const uint32_t i = SW::at(b0 | t2), j = SW::at(b0 | t1);
+    const uint32_t i = b0 | t2, j = b0 | t1;
     const double r = sre[i], q = sim[i];
     sre[i] = sre[j]; sim[i] = sim[j];
     sre[j] = r; sim[j] = q;
   }
 }
 
-template <class G, class SW = NoSwizzle>
+template <class G>
 __device__ __forceinline__ void tile_swap_any(const G& g, double* sre, double* sim, uint32_t nw) {
-#define SPZ_CALL(N) tile_swap<N, G, SW>(g, sre, sim, nw)
+#define SPZ_CALL(N) tile_swap<N, G>(g, sre, sim, nw)
   SPZ_BY_NPOS(g.npos, SPZ_CALL)
 #undef SPZ_CALL
 }
