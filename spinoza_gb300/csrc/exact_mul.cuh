@@ -126,4 +126,21 @@ SPZ_HD uint64_t mul_int(uint64_t y, const MulCoef& c) {
 #endif
 }
 
+// |y| * |y| rounded, as bits, for sqr_ok(y): mul_int with the coefficient made
+// from y itself.
+SPZ_HD bool sqr_ok(uint64_t y) {
+  // exponents e with 2 <= 2 e - 1023 <= 2044
+  return (((uint32_t)(y >> 32) & 0x7FFFFFFFu) - (513u << 20)) < ((1533u - 513u) << 20);
+}
+
+SPZ_HD uint64_t sqr_int(uint64_t y) {
+  y &= 0x7FFFFFFFFFFFFFFFull;
+  const uint32_t hi = (uint32_t)(y >> 32), lo = (uint32_t)y;
+  MulCoef m;
+  m.ch = (((hi & 0x000FFFFFu) | 0x00100000u) << 10) | (lo >> 22);
+  m.cl = lo << 10;
+  m.kexp = (hi & 0x7FF00000u) - (1022u << 20);
+  return mul_int(y, m);
+}
+
 }  // namespace spz
