@@ -7,6 +7,7 @@ fuses runs of gates into shared-memory tile passes.
 from __future__ import annotations
 
 import math
+import struct
 from ctypes import byref
 from typing import Iterable, List, Optional, Sequence, Set
 
@@ -120,26 +121,40 @@ class QubitTracker:
         return int((self.c.values >> q) & 1) if self.is_qubit_measured(q) else None
 
 
+_OP = struct.Struct("<iIIIdddIiQQ")  # one OP_DTYPE record
+assert _OP.size == nat.OP_DTYPE.itemsize
+
+
 def _ops_array(transformations: Sequence[QuantumTransformation], draws) -> np.ndarray:
-    ops = np.zeros(len(transformations), dtype=nat.OP_DTYPE)
-    for i, tr in enumerate(transformations):
+    """The C-ABI records of the transformations, packed one by one into a byte
+    buffer (a record costs about 1 us; assigning it to a structured array 3)."""
+    buf = bytearray(_OP.size * len(transformations))
+    pos = 0
+    for tr in transformations:
         g = tr.gate
-        if g.kind == nat.UNITARY:
+        kind = g.kind
+        p0, p1, p2 = g.params
+        if kind == nat.UNITARY:
             raise nat.Unsupported(nat.SPZ_ERR_UNSUPPORTED, "a dense Unitary is not an op; QuantumCircuit.execute "
                                                           "applies it between op runs")
-        p = list(g.params)
-        if g.kind == nat.M:
-            p[0] = draws()
-        elif g.kind == nat.BITFLIP and math.isnan(p[1]):
-            p[1] = next_noise_draw()
-        cmask = 0
-        for c in tr.controls.controls:
-            cmask |= 1 << c
-        zmask = 0
-        for z in tr.controls.zeros:
-            zmask |= 1 << z
-        ops[i] = ((g.kind, g.qubits[0], g.qubits[1], 0, p), tr.target, tr.controls.kind, cmask, zmask)
-    return ops
+        if kind == nat.M:
+            p0 = draws()
+        elif kind == nat.BITFLIP and math.isnan(p1):
+            p1 = next_noise_draw()
+        c = tr.controls
+        cmask = zmask = 0
+        for q in c.controls:
+            cmask |= 1 << q
+        for q in c.zeros:
+            zmask |= 1 << q
+        row = (kind, g.qubits[0], g.qubits[1], 0, p0, p1, p2, tr.target, c.kind, cmask, zmask)
+        try:
+            _OP.pack_into(buf, pos, *row)
+        except struct.error:  # a number outside its field: numpy says which
+            np.zeros(1, dtype=nat.OP_DTYPE)[0] = (row[:4] + (row[4:7],),) + row[7:]
+            raise
+        pos += _OP.size
+    return np.frombuffer(buf, dtype=nat.OP_DTYPE)
 
 
 class QuantumCircuit:
@@ -261,7 +276,7 @@ class QuantumCircuit:
 
     # execution
     def _next_draw(self) -> float:
-        u = float(rng.uniforms(self._seed, 1, self._draw_index)[0])
+        u = rng.uniform(self._seed, self._draw_index)
         self._draw_index += 1
         return u
 

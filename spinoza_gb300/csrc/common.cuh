@@ -93,6 +93,7 @@ struct spz_state_s {
   bool owns = false;
   cudaStream_t own_stream = nullptr;
   cudaStream_t stream = nullptr;
+  bool shared = false;  // the arrays may have been used on a stream other than own_stream
   int device = 0;
   // Reduction / planning scratch, grown on demand and reused.
   spz::Scratch dev_scratch;

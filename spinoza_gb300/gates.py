@@ -26,10 +26,16 @@ class Gate:
 
     def __init__(self, kind: int, params: Sequence[float] = (), qubits: Sequence[int] = (), matrix=None):
         self.kind = int(kind)
-        p = [float(v) for v in params] + [0.0] * (3 - len(params))
-        self.params = tuple(p[:3])
-        q = [int(v) for v in qubits] + [0] * (2 - len(qubits))
-        self.qubits = tuple(q[:2])
+        if len(params) == 1:
+            self.params = (float(params[0]), 0.0, 0.0)
+        else:
+            p = [float(v) for v in params] + [0.0] * (3 - len(params))
+            self.params = tuple(p[:3])
+        if qubits:
+            q = [int(v) for v in qubits] + [0] * (2 - len(qubits))
+            self.qubits = tuple(q[:2])
+        else:
+            self.qubits = (0, 0)
         self.matrix = matrix  # Unitary payload (gates.rs:67)
 
     @staticmethod
@@ -153,7 +159,7 @@ def seed_noise(seed: int) -> None:
 def next_noise_draw() -> float:
     from . import rng
 
-    u = float(rng.uniforms(_flip_stream[0], 1, _flip_stream[1])[0])
+    u = rng.uniform(_flip_stream[0], _flip_stream[1])
     _flip_stream[1] += 1
     return u
 

@@ -17,7 +17,7 @@ def seed_measurements(seed: int) -> None:
 
 
 def next_draw() -> float:
-    u = float(rng.uniforms(_stream[0], 1, _stream[1])[0])
+    u = rng.uniform(_stream[0], _stream[1])
     _stream[1] += 1
     return u
 
