@@ -65,26 +65,108 @@ __global__ void adj_finalize_kernel(const double* __restrict__ partials, int nbl
 
 enum GradMode { GM_X = 0, GM_Y = 1, GM_Z = 2, GM_P1 = 3 };
 
-// lam = D psi for the diagonal terms (or 0 when there are none).
-struct DiagSum {
-  int nterms;
-  double coeff[64];
-  uint64_t zmask[64];
+// lam = H psi in passes over tiles of 2^k amplitudes held in shared memory: the
+// first pass sets lam to the diagonal part plus every X/Y term whose X-mask lies
+// in its tile, later passes add theirs.  The diagonal part is 8-bit chunk tables
+// (as in pauli_tile_kernel, reduce.cu).  One pass per about eight X-masks instead
+// of one over the whole state per X-mask: 21 qubits, 20 ZZ and 21 X terms, 1078 us
+// in 22 launches -> 207 us in 3, near the DFMA rate (2 per X term and amplitude).
+constexpr int kHpK = 11, kHpLow = 3, kHpThreads = 256, kHpMaxTerms = 32, kHpMaxDiag = 64;
+
+struct HpTerm {
+  double cr, ci;  // c i^ny
+  uint64_t z;     // Z-mask (qubits)
+  uint32_t xl;    // X-mask as bits of the tile offset
+  int32_t plain;  // z = 0: the coefficient is cr for every amplitude
 };
 
-__global__ void hamiltonian_diag_kernel(const double* __restrict__ pr, const double* __restrict__ pi,
-                                        double* __restrict__ lr, double* __restrict__ li, uint64_t N, DiagSum T) {
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t x = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; x < N; x += stride) {
-    double dsum = 0.0;
-    for (int k = 0; k < T.nterms; ++k)
-      dsum = dadd(dsum, (__popcll(x & T.zmask[k]) & 1) ? dneg(T.coeff[k]) : T.coeff[k]);
-    lr[x] = dmul(dsum, pr[x]);
-    li[x] = dmul(dsum, pi[x]);
+struct HpArgs {
+  const double* pr;
+  const double* pi;
+  double* lr;
+  double* li;
+  uint64_t ntiles;
+  int k, c, nhigh, first, nt, nch, ndiag;
+  uint8_t lpos[kHpK + 1];
+  const double* dtab;                    // nch x 256 entries
+  uint64_t dz[kHpMaxDiag];
+  uint8_t lz[kHpMaxDiag / 8][2][64];     // chunk index of tile-offset bits 0-5 and 6-11
+  HpTerm t[kHpMaxTerms];
+};
+
+__global__ void __launch_bounds__(kHpThreads) hamiltonian_tile_kernel(const __grid_constant__ HpArgs A) {
+  extern __shared__ double sm[];
+  const uint32_t T = 1u << A.k;
+  double* sre = sm;
+  double* sim = sm + T;
+  uint64_t* rowoff = reinterpret_cast<uint64_t*>(sm + 2 * T);
+  double* stab = sm + 2 * T + (1u << A.nhigh);
+  uint8_t* slz = reinterpret_cast<uint8_t*>(stab + (size_t)A.nch * 256);
+  const uint32_t cmask = (1u << A.c) - 1;
+  for (uint32_t r = threadIdx.x; r < (1u << A.nhigh); r += blockDim.x)
+    rowoff[r] = row_offset_param<kHpK>(r, A.lpos, A.c, A.k);
+  for (int j = threadIdx.x; j < A.nch * 256; j += blockDim.x) stab[j] = A.dtab[j];
+  for (int j = threadIdx.x; j < A.nch * 128; j += blockDim.x) slz[j] = (&A.lz[0][0][0])[j];
+  __syncthreads();
+  for (uint64_t tile = blockIdx.x; tile < A.ntiles; tile += gridDim.x) {
+    const uint64_t base = deposit_param<kHpK>(tile, A.lpos, A.k);
+    for (uint32_t e2 = threadIdx.x; e2 < T / 2; e2 += blockDim.x) {
+      const uint32_t e = 2 * e2;
+      const uint64_t gi = base | rowoff[e >> A.c] | (e & cmask);
+      *reinterpret_cast<double2*>(sre + e) = *reinterpret_cast<const double2*>(A.pr + gi);
+      *reinterpret_cast<double2*>(sim + e) = *reinterpret_cast<const double2*>(A.pi + gi);
+    }
+    uint32_t wb[kHpMaxDiag / 8];  // the tile base's part of each chunk index
+#pragma unroll
+    for (int ch = 0; ch < kHpMaxDiag / 8; ++ch) {
+      wb[ch] = 0;
+      if (ch < A.nch)
+        for (int j = 0; j < min(8, A.ndiag - ch * 8); ++j)
+          wb[ch] |= (uint32_t)(__popcll(base & A.dz[ch * 8 + j]) & 1) << j;
+    }
+    __syncthreads();
+    for (uint32_t e = threadIdx.x; e < T; e += blockDim.x) {
+      const uint64_t gi = base | rowoff[e >> A.c] | (e & cmask);
+      double dr, di;
+      if (A.first) {
+        double d = 0.0;
+        const uint32_t e0 = e & 63, e1 = e >> 6;
+#pragma unroll
+        for (int ch = 0; ch < kHpMaxDiag / 8; ++ch) {
+          if (ch >= A.nch) break;
+          const double v = stab[ch * 256 + (wb[ch] ^ slz[ch * 128 + e0] ^ slz[ch * 128 + 64 + e1])];
+          d = ch == 0 ? v : dadd(d, v);
+        }
+        dr = dmul(d, sre[e]);
+        di = dmul(d, sim[e]);
+      } else {
+        dr = A.lr[gi];
+        di = A.li[gi];
+      }
+      for (int t = 0; t < A.nt; ++t) {
+        const HpTerm& P = A.t[t];
+        const uint32_t y = e ^ P.xl;
+        const double yr = sre[y], yi = sim[y];
+        if (P.plain) {
+          dr = dfma(P.cr, yr, dr);
+          di = dfma(P.cr, yi, di);
+        } else {
+          const uint64_t gy = base | rowoff[y >> A.c] | (y & cmask);
+          const bool neg = (__popcll(gy & P.z) & 1) != 0;
+          const double cr = neg ? dneg(P.cr) : P.cr, ci = neg ? dneg(P.ci) : P.ci;
+          dr = dfma(cr, yr, dfma(dneg(ci), yi, dr));
+          di = dfma(cr, yi, dfma(ci, yr, di));
+        }
+      }
+      A.lr[gi] = dr;
+      A.li[gi] = di;
+    }
+    __syncthreads();
   }
 }
 
-// lam_x += sum_k c_k i^ny_k (-1)^popc(y & z_k) psi_y,  y = x ^ xmask.
+// lam_x += sum_k c_k i^ny_k (-1)^popc(y & z_k) psi_y,  y = x ^ xmask, for an X-mask
+// wider than a tile.
 struct XSum {
   int nterms;
   uint64_t xmask;
@@ -127,13 +209,20 @@ __global__ void inner_re_kernel(const double* __restrict__ pr, const double* __r
 #ifndef SPZ_ADJ_TILE_K
 #define SPZ_ADJ_TILE_K 10
 #endif
+// 128 threads x 6 blocks per SM (what the tiles' shared memory allows): with the
+// products on the integer pipes 12 warps per SM (64 threads) no longer fill the
+// FP64 pipe.  21 qubits, 6 layers, the six passes: 15.2 ms with DFMA products and
+// 64 threads, 10.8 ms now.
 #ifndef SPZ_ADJ_THREADS
-#define SPZ_ADJ_THREADS 64
+#define SPZ_ADJ_THREADS 128
+#endif
+#ifndef SPZ_ADJ_MIN_BLOCKS
+#define SPZ_ADJ_MIN_BLOCKS 6
 #endif
 constexpr int kAdjTileK = SPZ_ADJ_TILE_K;  // psi and lam tiles: 4 x 2^10 doubles = 32 KiB
 constexpr int kAdjTileThreads = SPZ_ADJ_THREADS;
 constexpr int kAdjWarps = kAdjTileThreads / 32;
-constexpr int kAdjMaxSlots = 256;   // differentiated gates per backward pass
+constexpr int kAdjMaxSlots = 128;   // differentiated gates per backward pass
 
 struct AdjOp {
   int32_t mode;  // GradMode, or -1: no gradient at this gate
@@ -157,14 +246,22 @@ struct AdjPassArgs {
   uint8_t lpos[16];
 };
 
-// Gradient term of one pair / element, as in grad_pair_kernel.
-__device__ __forceinline__ double adj_pair_term(int mode, double a, double b, double c, double d, double p, double q,
-                                                double r, double s) {
+// Adds one pair's gradient term to acc: four FMAs (two for P1) instead of a sum
+// of products and an add.
+__device__ __forceinline__ void adj_pair_term(int mode, double a, double b, double c, double d, double p, double q,
+                                              double r, double s, double& x, double& y) {
   switch (mode) {
-    case GM_X: return dadd(dfma(p, d, dmul(dneg(q), c)), dfma(r, b, dmul(dneg(s), a)));
-    case GM_Y: return dsub(dfma(r, a, dmul(s, b)), dfma(p, c, dmul(q, d)));
-    case GM_Z: return dsub(dfma(p, b, dmul(dneg(q), a)), dfma(r, d, dmul(dneg(s), c)));
-    default: return dfma(r, d, dmul(dneg(s), c));
+    case GM_X:  // (p d - q c) + (r b - s a)
+      x = dfma(p, d, x); y = dfma(dneg(q), c, y); x = dfma(r, b, x); y = dfma(dneg(s), a, y);
+      break;
+    case GM_Y:  // (r a + s b) - (p c + q d)
+      x = dfma(r, a, x); y = dfma(dneg(p), c, y); x = dfma(s, b, x); y = dfma(dneg(q), d, y);
+      break;
+    case GM_Z:  // (p b - q a) - (r d - s c)
+      x = dfma(p, b, x); y = dfma(dneg(q), a, y); x = dfma(s, c, x); y = dfma(dneg(r), d, y);
+      break;
+    default:  // r d - s c
+      x = dfma(r, d, x); y = dfma(dneg(s), c, y);
   }
 }
 
@@ -175,18 +272,18 @@ __device__ __forceinline__ double adj_pair(const TileGate& g, int mode, double* 
   const Enumerator<NPOS, TileGate> E(g);
   const uint32_t tbit = g.tbit;
   const PairGate<KIND> op(g.c);
-  double acc = 0.0;
+  double x = 0.0, y = 0.0;
   for (uint32_t m = threadIdx.x; m < nw; m += blockDim.x) {
     const uint32_t s0 = E(m), s1 = s0 | tbit;
     double a = pr[s0], b = pi[s0], c = pr[s1], d = pi[s1];
     double p = lr[s0], q = li[s0], r = lr[s1], s = li[s1];
-    if (mode >= 0) acc = dadd(acc, adj_pair_term(mode, a, b, c, d, p, q, r, s));
+    if (mode >= 0) adj_pair_term(mode, a, b, c, d, p, q, r, s, x, y);
     op(a, b, c, d);
     op(p, q, r, s);
     pr[s0] = a; pi[s0] = b; pr[s1] = c; pi[s1] = d;
     lr[s0] = p; li[s0] = q; lr[s1] = r; li[s1] = s;
   }
-  return acc;
+  return dadd(x, y);
 }
 
 // Diagonal gates (Z, P, RZ): elementwise; the target bit comes from the
@@ -199,20 +296,21 @@ __device__ __forceinline__ double adj_diag(const TileGate& g, int mode, int glob
   const Enumerator<NPOS, TileGate> E(g);
   const uint32_t tbit = g.tbit;
   const DiagGate<KIND> op(g.c);
-  double acc = 0.0;
+  double x = 0.0, y = 0.0;
   for (uint32_t m = threadIdx.x; m < nw; m += blockDim.x) {
     const uint32_t e = E(m);
     const bool one = global_one >= 0 ? global_one != 0 : (e & tbit) != 0;
     double a = pr[e], b = pi[e], p = lr[e], q = li[e];
     if (mode >= 0) {
-      const double v = dfma(p, b, dmul(dneg(q), a));  // Im(conj(lam) psi)
-      acc = (mode == GM_Z && one) ? dsub(acc, v) : dadd(acc, v);
+      const bool minus = mode == GM_Z && one;  // +- Im(conj(lam) psi)
+      x = dfma(minus ? dneg(p) : p, b, x);
+      y = dfma(minus ? q : dneg(q), a, y);
     }
     op(one, a, b);
     op(one, p, q);
     pr[e] = a; pi[e] = b; lr[e] = p; li[e] = q;
   }
-  return acc;
+  return dadd(x, y);
 }
 
 template <int KIND>
@@ -235,7 +333,7 @@ __device__ __forceinline__ double adj_diag_any(const TileGate& g, int mode, int 
   return r;
 }
 
-__global__ void __launch_bounds__(kAdjTileThreads) adj_tile_kernel(const __grid_constant__ AdjPassArgs A) {
+__global__ void __launch_bounds__(kAdjTileThreads, SPZ_ADJ_MIN_BLOCKS) adj_tile_kernel(const __grid_constant__ AdjPassArgs A) {
   extern __shared__ double sm[];
   const int K = A.k;
   const uint32_t T = 1u << K;
@@ -360,6 +458,130 @@ int ensure_aux(spz_state_t h, int j) {
   return SPZ_OK;
 }
 
+// lam = H psi (psi in the handle).
+int apply_hamiltonian(spz_state_t h, const spz_pauli_term* terms, size_t nterms, double* lr, double* li) {
+  const int n = (int)h->n, k = std::min(n, kHpK), c = std::min(kHpLow, k);
+  std::vector<size_t> diag, xt, wide;
+  for (size_t j = 0; j < nterms; ++j) {
+    if (terms[j].x_mask == 0) diag.push_back(j);
+    else (__builtin_popcountll(terms[j].x_mask & ~((1ull << c) - 1)) <= k - c ? xt : wide).push_back(j);
+  }
+  if (diag.size() > (size_t)kHpMaxDiag) return fail(SPZ_ERR_UNSUPPORTED, "more than 64 diagonal terms");
+  const size_t nch = (diag.size() + 7) / 8;
+  // Entry v of a chunk: sum of its coefficients, negated where v has the bit.  (Not
+  // a constant plus corrections: the constant's rounding would shift every
+  // amplitude's value alike, and with it the energy.)
+  std::vector<double> tab(std::max<size_t>(1, nch * 256), 0.0);
+  for (size_t ch = 0; ch < nch; ++ch)
+    for (int v = 0; v < 256; ++v) {
+      double hi = 0.0, lo = 0.0;
+      for (int b = 0; b < 8 && ch * 8 + b < diag.size(); ++b) {
+        const double c = ((v >> b) & 1) ? -terms[diag[ch * 8 + b]].coeff : terms[diag[ch * 8 + b]].coeff;
+        const double t = hi + c, z = t - hi;  // two-sum
+        lo += (hi - (t - z)) + (c - z);
+        hi = t;
+      }
+      tab[ch * 256 + v] = hi + lo;
+    }
+  void* scratch;
+  int rc = ensure_dev_scratch(h, tab.size() * sizeof(double), &scratch);
+  if (rc) return rc;
+  SPZ_CUDA(cudaMemcpyAsync(scratch, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+  {  // the shared-memory opt-in, once per device
+    static std::mutex mu;
+    static bool ready[kMaxDevices] = {};
+    if (h->device < 0 || h->device >= kMaxDevices) return fail(SPZ_ERR_INVALID_ARGUMENT, "device index out of range");
+    std::lock_guard<std::mutex> lock(mu);
+    if (!ready[h->device]) {
+      const size_t most = ((2u << kHpK) + (1u << (kHpK - kHpLow)) + (kHpMaxDiag / 8) * (256 + 16)) * sizeof(double);
+      SPZ_CUDA(cudaFuncSetAttribute(hamiltonian_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+      ready[h->device] = true;
+    }
+  }
+  std::vector<bool> done(xt.size(), false);
+  size_t left = xt.size();
+  for (bool first = true; first || left; first = false) {
+    HpArgs A{};
+    uint64_t L = (1ull << c) - 1;
+    std::vector<size_t> take;
+    for (size_t j = 0; j < xt.size() && (int)take.size() < kHpMaxTerms; ++j) {
+      const uint64_t with = L | terms[xt[j]].x_mask;
+      if (done[j] || __builtin_popcountll(with) > k) continue;
+      L = with;
+      done[j] = true;
+      take.push_back(xt[j]);
+      --left;
+    }
+    for (int q = 0; q < n && __builtin_popcountll(L) < k; ++q) L |= 1ull << q;
+    int where[64] = {};
+    for (int q = 0; q < n; ++q)
+      if ((L >> q) & 1) {
+        where[q] = A.k;
+        A.lpos[A.k++] = (uint8_t)q;
+      }
+    A.pr = h->re;
+    A.pi = h->im;
+    A.lr = lr;
+    A.li = li;
+    A.ntiles = 1ull << (n - A.k);
+    A.c = c;
+    A.nhigh = A.k - c;
+    A.first = first;
+    A.nt = (int)take.size();
+    for (int t = 0; t < A.nt; ++t) {
+      const spz_pauli_term& m = terms[take[t]];
+      const int ny = __builtin_popcountll(m.x_mask & m.z_mask) & 3;
+      const double v = ny >= 2 ? -m.coeff : m.coeff;
+      A.t[t].cr = (ny & 1) ? 0.0 : v;
+      A.t[t].ci = (ny & 1) ? v : 0.0;
+      A.t[t].z = m.z_mask;
+      A.t[t].plain = m.z_mask == 0;
+      for (int q = 0; q < n; ++q)
+        if ((m.x_mask >> q) & 1) A.t[t].xl |= 1u << where[q];
+    }
+    if (first) {
+      A.nch = (int)nch;
+      A.ndiag = (int)diag.size();
+      A.dtab = (const double*)scratch;
+      for (size_t j = 0; j < diag.size(); ++j) A.dz[j] = terms[diag[j]].z_mask;
+      for (int ch = 0; ch < A.nch; ++ch)
+        for (int v = 0; v < 64; ++v)
+          for (int b = 0; b < 6; ++b) {
+            if (!((v >> b) & 1)) continue;
+            for (int half = 0; half < 2; ++half) {
+              const int bit = b + 6 * half;
+              if (bit >= A.k) continue;
+              for (int j = 0; j < std::min(8, A.ndiag - ch * 8); ++j)
+                A.lz[ch][half][v] ^= (uint8_t)(((A.dz[ch * 8 + j] >> A.lpos[bit]) & 1) << j);
+            }
+          }
+    }
+    const size_t smem = ((2u << A.k) + (1u << A.nhigh) + (size_t)A.nch * (256 + 16)) * sizeof(double);
+    const int blocks = (int)std::min<uint64_t>(A.ntiles, (uint64_t)kNumSMs * 6);
+    const int threads = (int)std::min<uint32_t>(kHpThreads, std::max<uint32_t>(32, (1u << A.k) / 2));
+    hamiltonian_tile_kernel<<<blocks, threads, smem, h->stream>>>(A);
+    SPZ_CHECK_LAUNCH("hamiltonian_tile_kernel");
+  }
+  while (!wide.empty()) {
+    XSum X{};
+    X.xmask = terms[wide[0]].x_mask;
+    std::vector<size_t> rest;
+    for (size_t j : wide) {
+      if (terms[j].x_mask != X.xmask || X.nterms == 64) {
+        rest.push_back(j);
+        continue;
+      }
+      X.coeff[X.nterms] = terms[j].coeff;
+      X.zmask[X.nterms] = terms[j].z_mask;
+      X.ny[X.nterms++] = __builtin_popcountll(terms[j].x_mask & terms[j].z_mask);
+    }
+    wide.swap(rest);
+    hamiltonian_x_kernel<<<grid_for(h->N), kThreads, 0, h->stream>>>(h->re, h->im, lr, li, h->N, X);
+    SPZ_CHECK_LAUNCH("hamiltonian_x_kernel");
+  }
+  return SPZ_OK;
+}
+
 // Inverse of a gate (gates.rs:80-92: angle negation; U(t,p,l)^-1 = U(-t,-l,-p)).
 spz_gate inverse_gate(const spz_gate& g) {
   spz_gate r = g;
@@ -447,36 +669,8 @@ int adjoint_gradient(spz_state_t h, const spz_op* ops, size_t nops, const uint32
   if (rc) return rc;
   double *lr = h->aux_re[0], *li = h->aux_im[0], *wr = h->aux_re[1], *wi = h->aux_im[1];
   // lam = H psi.
-  std::vector<std::vector<size_t>> groups;
-  std::vector<uint64_t> gx;
-  for (size_t k = 0; k < nterms; ++k) {
-    size_t g = 0;
-    for (; g < groups.size(); ++g)
-      if (gx[g] == terms[k].x_mask && groups[g].size() < 64) break;
-    if (g == groups.size()) { groups.emplace_back(); gx.push_back(terms[k].x_mask); }
-    groups[g].push_back(k);
-  }
-  DiagSum D{};
-  for (size_t g = 0; g < groups.size(); ++g)
-    if (gx[g] == 0)
-      for (size_t k : groups[g]) {
-        if (D.nterms == 64) return fail(SPZ_ERR_UNSUPPORTED, "more than 64 diagonal terms");
-        D.coeff[D.nterms] = terms[k].coeff;
-        D.zmask[D.nterms++] = terms[k].z_mask;
-      }
-  hamiltonian_diag_kernel<<<grid_for(h->N), kThreads, 0, h->stream>>>(h->re, h->im, lr, li, h->N, D);
-  for (size_t g = 0; g < groups.size(); ++g) {
-    if (gx[g] == 0) continue;
-    XSum X{};
-    X.xmask = gx[g];
-    for (size_t k : groups[g]) {
-      X.coeff[X.nterms] = terms[k].coeff;
-      X.zmask[X.nterms] = terms[k].z_mask;
-      X.ny[X.nterms++] = __builtin_popcountll(terms[k].x_mask & terms[k].z_mask);
-    }
-    hamiltonian_x_kernel<<<grid_for(h->N), kThreads, 0, h->stream>>>(h->re, h->im, lr, li, h->N, X);
-  }
-  SPZ_CHECK_LAUNCH("hamiltonian kernels");
+  rc = apply_hamiltonian(h, terms, nterms, lr, li);
+  if (rc) return rc;
   // Backward: the inverse gates in reverse order, fused into tile passes
   // (passes with more than kAdjMaxSlots differentiated gates are cut).
   std::vector<GateApp> bwd;

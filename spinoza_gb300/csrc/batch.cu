@@ -232,27 +232,24 @@ __device__ __forceinline__ double b_bwd_pair(const BGate& g, double* pr, double*
   const uint32_t tbit = g.tbit;
   const PairGate<KIND> op(g.c);
   const int grad = g.grad;
-  double acc = 0.0;
+  double x = 0.0, y = 0.0;
   for (uint32_t m = threadIdx.x; m < nw; m += blockDim.x) {
     const uint32_t s0 = E(m), s1 = s0 | tbit;
     double a = pr[s0], b = pi[s0], c = pr[s1], d = pi[s1];
     double p = lr[s0], q = li[s0], r = lr[s1], s = li[s1];
-    if (grad != BG_NONE) {
-      double v;
-      switch (grad) {
-        case BG_X: v = dadd(dfma(p, d, dmul(dneg(q), c)), dfma(r, b, dmul(dneg(s), a))); break;
-        case BG_Y: v = dsub(dfma(r, a, dmul(s, b)), dfma(p, c, dmul(q, d))); break;
-        case BG_Z: v = dsub(dfma(p, b, dmul(dneg(q), a)), dfma(r, d, dmul(dneg(s), c))); break;
-        default: v = dfma(r, d, dmul(dneg(s), c)); break;
-      }
-      acc = dadd(acc, v);
+    switch (grad) {  // FMA chains, as in the fused adjoint sweep
+      case BG_NONE: break;
+      case BG_X: x = dfma(p, d, x); y = dfma(dneg(q), c, y); x = dfma(r, b, x); y = dfma(dneg(s), a, y); break;
+      case BG_Y: x = dfma(r, a, x); y = dfma(dneg(p), c, y); x = dfma(s, b, x); y = dfma(dneg(q), d, y); break;
+      case BG_Z: x = dfma(p, b, x); y = dfma(dneg(q), a, y); x = dfma(s, c, x); y = dfma(dneg(r), d, y); break;
+      default: x = dfma(r, d, x); y = dfma(dneg(s), c, y);
     }
     op(a, b, c, d);
     op(p, q, r, s);
     pr[s0] = a; pi[s0] = b; pr[s1] = c; pi[s1] = d;
     lr[s0] = p; li[s0] = q; lr[s1] = r; li[s1] = s;
   }
-  return acc;
+  return dadd(x, y);
 }
 
 template <int KIND, int NPOS>
@@ -262,20 +259,21 @@ __device__ __forceinline__ double b_bwd_diag(const BGate& g, int gone, double* p
   const uint32_t tbit = g.tbit;
   const DiagGate<KIND> op(g.c);
   const int grad = g.grad;
-  double acc = 0.0;
+  double x = 0.0, y = 0.0;
   for (uint32_t m = threadIdx.x; m < nw; m += blockDim.x) {
     const uint32_t e = E(m);
     const bool one = gone >= 0 ? gone != 0 : (e & tbit) != 0;
     double a = pr[e], b = pi[e], p = lr[e], q = li[e];
     if (grad != BG_NONE && !(grad == BG_P1 && !one)) {
-      const double v = dfma(p, b, dmul(dneg(q), a));  // Im(conj(lam) psi)
-      acc = (grad == BG_Z && one) ? dsub(acc, v) : dadd(acc, v);
+      const bool minus = grad == BG_Z && one;  // +- Im(conj(lam) psi)
+      x = dfma(minus ? dneg(p) : p, b, x);
+      y = dfma(minus ? q : dneg(q), a, y);
     }
     op(one, a, b);
     op(one, p, q);
     pr[e] = a; pi[e] = b; lr[e] = p; li[e] = q;
   }
-  return acc;
+  return dadd(x, y);
 }
 
 template <int KIND>
@@ -1343,6 +1341,7 @@ int spz_batch_run(spz_batch_t b, const double* theta, double* energies, double* 
       }
       SPZ_CUDA(cudaStreamSynchronize(h->stream));  // its |0...0> fill ran on its own stream
       h->stream = b->wide_stream[si];
+      h->shared = true;
     }
     for (size_t j = 0; j < w.pidx.size(); ++j) w.ops[w.pidx[j]].gate.p[0] = theta[w.param_offset + j];
     int rc = spz_state_reset_zero(h);
