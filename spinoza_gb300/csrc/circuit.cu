@@ -1039,8 +1039,8 @@ size_t mark_shuffle_runs(TileGate* g, size_t count, int k) {
   return in_runs;
 }
 
-// Fast mode: fuse consecutive lazy rotations on two distinct tile qubits,
-// both carrying a phase entry, into one TM_LAZY2 op, when the second op's
+// Fast mode: fuse consecutive lazy rotations on two distinct tile qubits
+// into one TM_LAZY2 op, when the second op's
 // phase masks do not contain the first op's qubit (its phase then commutes
 // with the first rotation) and the two tables have at most kPhaseMaxTerms
 // masks between them.  pg[i] is the descriptor of gates[i]; the joint tables
@@ -1055,9 +1055,66 @@ bool fast_pairs_enabled() {
   return on;
 }
 
-bool lazy_with_table(const GateApp& g) {
-  return g.kind >= FK_LAZY_H && g.kind <= FK_LAZY_RY_B && g.table >= 0 && g.cond < 0 && g.ones == 0 &&
-         g.zeros == 0;
+bool lazy_uncontrolled(const GateApp& g) {
+  return g.kind >= FK_LAZY_H && g.kind <= FK_LAZY_RY_B && g.cond < 0 && g.ones == 0 && g.zeros == 0;
+}
+
+// A lazy op's phase table; without one, the single entry 1.
+const PhaseTable& table_of(const GateApp& g, const std::vector<PhaseTable>& tables) {
+  static const PhaseTable unit = [] {
+    PhaseTable t;
+    t.re = {1.0};
+    t.im = {0.0};
+    return t;
+  }();
+  return g.table >= 0 ? tables[g.table] : unit;
+}
+
+// Whether b can follow a in one TM_LAZY2 op.
+bool lazy_pair_fits(const GateApp& a, const GateApp& b, const std::vector<PhaseTable>& tables) {
+  if (!lazy_uncontrolled(a) || !lazy_uncontrolled(b) || a.target == b.target) return false;
+  const PhaseTable &T1 = table_of(a, tables), &T2 = table_of(b, tables);
+  bool ok = T1.m + T2.m <= kPhaseMaxTerms;
+  for (int j = 0; ok && j < T2.m; ++j) ok = ((T2.mask[j] >> a.target) & 1) == 0;
+  return ok;
+}
+
+// Reorder a pass's gates (any two that commute) so that lazy ops that fit
+// together stand side by side: a partner further on moves up to its lazy op, or
+// the lazy op down to it.  (30-qubit brickwork, 20 layers: 269 pairs instead of
+// 261; few more fit, a layer's gates inside one pass being an odd number.)
+void order_lazy_pairs(std::vector<GateApp>* gates, const std::vector<PhaseTable>& tables) {
+  if (!fast_pairs_enabled()) return;
+  std::vector<GateApp>& g = *gates;
+  auto commute = [](const GateApp& a, const GateApp& b) {
+    return (nd_mask(a) & (nd_mask(b) | d_mask(b))) == 0 && (d_mask(a) & nd_mask(b)) == 0;
+  };
+  constexpr size_t kReach = 64;
+  for (size_t i = 0; i + 1 < g.size(); ++i) {
+    if (!lazy_uncontrolled(g[i])) continue;
+    if (lazy_pair_fits(g[i], g[i + 1], tables)) {
+      ++i;
+      continue;
+    }
+    for (size_t j = i + 2; j < g.size() && j < i + kReach; ++j) {
+      if (!lazy_pair_fits(g[i], g[j], tables)) continue;
+      bool up = true, down = true;
+      for (size_t b = i + 1; b < j; ++b) {
+        up = up && commute(g[j], g[b]);
+        down = down && commute(g[i], g[b]);
+      }
+      if (up) {
+        std::rotate(g.begin() + (ptrdiff_t)i + 1, g.begin() + (ptrdiff_t)j, g.begin() + (ptrdiff_t)j + 1);
+        ++i;
+        break;
+      }
+      if (down) {
+        std::rotate(g.begin() + (ptrdiff_t)i, g.begin() + (ptrdiff_t)i + 1, g.begin() + (ptrdiff_t)j);
+        --i;  // the gate now at i has not been looked at
+        break;
+      }
+    }
+  }
 }
 
 uint64_t fuse_lazy_pairs(std::vector<TileGate>& pg, const std::vector<GateApp>& gates,
@@ -1067,55 +1124,49 @@ uint64_t fuse_lazy_pairs(std::vector<TileGate>& pg, const std::vector<GateApp>& 
   uint64_t saved = 0;
   size_t i = 0;
   while (i < pg.size()) {
-    if (i + 1 < pg.size() && lazy_with_table(gates[i]) && lazy_with_table(gates[i + 1]) &&
-        gates[i].target != gates[i + 1].target && pg[i].mode == TM_PAIR && pg[i + 1].mode == TM_PAIR) {
-      const PhaseTable& T1 = tables[gates[i].table];
-      const PhaseTable& T2 = tables[gates[i + 1].table];
-      const uint64_t q1b = 1ull << gates[i].target, q2b = 1ull << gates[i + 1].target;
-      bool ok = T1.m + T2.m <= kPhaseMaxTerms;
-      for (int j = 0; ok && j < T2.m; ++j) ok = (T2.mask[j] & q1b) == 0;
-      if (ok) {
-        TileGate t = pg[i];
-        const TileGate& u = pg[i + 1];
-        t.mode = TM_LAZY2;
-        t.kind2 = u.kind;
-        t.tbit2 = u.tbit;
-        t.c.sn = u.c.cs;
-        const FxLazy x1 = fx_lazy(gates[i].kind, gates[i].c.cs), x2 = fx_lazy(gates[i + 1].kind, gates[i + 1].c.cs);
-        t.fx2 = u.fx1;
-        t.fxswaps = (x1.swap ? 1u : 0u) | (x2.swap ? 2u : 0u);
-        t.fxturns = 0;
-        for (int j = 0; j < 4; ++j) t.fxturns |= ((x1.turns(j & 1) + x2.turns(j >> 1)) & 3u) << (2 * j);
-        const int p1 = __builtin_ctz(t.tbit), p2 = __builtin_ctz(u.tbit);
-        t.npos = 2;
-        t.pos[0] = (uint8_t)std::min(p1, p2);
-        t.pos[1] = (uint8_t)std::max(p1, p2);
-        t.l_ones = 0;
-        t.e_mask = t.tbit | u.tbit;
-        t.pm1 = T1.m;
-        t.pm = T1.m + T2.m;
-        for (int j = 0; j < T2.m; ++j) {
-          t.pmask[T1.m + j] = u.pmask[j];
-          t.pemask[T1.m + j] = u.pemask[j];
-        }
-        uint32_t flip = 0;
-        for (int j = 0; j < T1.m; ++j)
-          if (T1.mask[j] & q2b) flip |= 1u << j;
-        t.ptab = (uint32_t)flat->entries.size();
-        const uint32_t E = 1u << t.pm;
-        for (uint32_t idx = 0; idx < E; ++idx) {
-          const uint32_t i1 = idx & ((1u << T1.m) - 1), i2 = idx >> T1.m;
-          const std::complex<double> w1(T1.re[i1], T1.im[i1]), w2(T2.re[i2], T2.im[i2]);
-          const std::complex<double> w3 = std::complex<double>(T1.re[i1 ^ flip], T1.im[i1 ^ flip]) * w2;
-          flat->push(w1, 0, x1.pre);
-          flat->push(w2, 0, x2.pre);
-          flat->push(w3, 0, x1.pre + x2.pre);
-        }
-        out.push_back(t);
-        saved += 1ull << n;
-        i += 2;
-        continue;
+    if (i + 1 < pg.size() && lazy_pair_fits(gates[i], gates[i + 1], tables)) {
+      const PhaseTable &T1 = table_of(gates[i], tables), &T2 = table_of(gates[i + 1], tables);
+      const uint64_t q2b = 1ull << gates[i + 1].target;
+      TileGate t = pg[i];
+      const TileGate& u = pg[i + 1];
+      t.mode = TM_LAZY2;
+      t.kind2 = u.kind;
+      t.tbit2 = u.tbit;
+      t.c.sn = u.c.cs;
+      const FxLazy x1 = fx_lazy(gates[i].kind, gates[i].c.cs), x2 = fx_lazy(gates[i + 1].kind, gates[i + 1].c.cs);
+      t.fx2 = u.fx1;
+      t.fxswaps = (x1.swap ? 1u : 0u) | (x2.swap ? 2u : 0u);
+      t.fxturns = 0;
+      for (int j = 0; j < 4; ++j) t.fxturns |= ((x1.turns(j & 1) + x2.turns(j >> 1)) & 3u) << (2 * j);
+      const int p1 = __builtin_ctz(t.tbit), p2 = __builtin_ctz(u.tbit);
+      t.npos = 2;
+      t.pos[0] = (uint8_t)std::min(p1, p2);
+      t.pos[1] = (uint8_t)std::max(p1, p2);
+      t.l_ones = 0;
+      t.e_mask = t.tbit | u.tbit;
+      t.pm1 = T1.m;
+      t.pm = T1.m + T2.m;
+      for (int j = 0; j < T2.m; ++j) {
+        t.pmask[T1.m + j] = u.pmask[j];
+        t.pemask[T1.m + j] = u.pemask[j];
       }
+      uint32_t flip = 0;
+      for (int j = 0; j < T1.m; ++j)
+        if (T1.mask[j] & q2b) flip |= 1u << j;
+      t.ptab = (uint32_t)flat->entries.size();
+      const uint32_t E = 1u << t.pm;
+      for (uint32_t idx = 0; idx < E; ++idx) {
+        const uint32_t i1 = idx & ((1u << T1.m) - 1), i2 = idx >> T1.m;
+        const std::complex<double> w1(T1.re[i1], T1.im[i1]), w2(T2.re[i2], T2.im[i2]);
+        const std::complex<double> w3 = std::complex<double>(T1.re[i1 ^ flip], T1.im[i1 ^ flip]) * w2;
+        flat->push(w1, 0, x1.pre);
+        flat->push(w2, 0, x2.pre);
+        flat->push(w3, 0, x1.pre + x2.pre);
+      }
+      out.push_back(t);
+      if (gates[i].table >= 0 && gates[i + 1].table >= 0) saved += 1ull << n;
+      i += 2;
+      continue;
     }
     out.push_back(pg[i]);
     ++i;
@@ -1493,6 +1544,8 @@ int run_gates_io(spz_state_t h, const std::vector<GateApp>& gates_in, uint32_t f
   const int c = std::min<int>(kTileLowBits, k);
   std::vector<PlannedPass> passes = plan(gates, n, k, c, !fast);
   pad_tile_passes(passes, n, k);
+  if (fast)
+    for (PlannedPass& P : passes) order_lazy_pairs(&P.gates, tables);
   // Phase tables, after the gate list.
   std::vector<uint32_t> table_offsets;
   FlatTables flat = flatten(gates, tables, &table_offsets);
@@ -1995,6 +2048,8 @@ int plan_stats(uint32_t n, const spz_op* ops, size_t nops, uint32_t flags, spz_e
       const std::vector<uint32_t> no_offsets(tables.size(), 0);
       std::vector<PlannedPass> planned = plan(run, n, k, c, !fast);
       pad_tile_passes(planned, n, k);
+      if (fast)
+        for (PlannedPass& P : planned) order_lazy_pairs(&P.gates, tables);
       FlatTables no_flat;
       for (const PlannedPass& P : planned) {
         const bool tiled = P.gates.size() > 1 || P.gates[0].kind >= FK_LAZY_H || P.gates[0].cond >= 0;
@@ -2143,6 +2198,8 @@ int build_program(spz_program_t p, const spz_op* ops, size_t nops, uint32_t flag
   const int c = std::min<int>(kTileLowBits, k);
   std::vector<PlannedPass> planned = plan(gates, n, k, c, !fast);
   pad_tile_passes(planned, n, k);
+  if (fast)
+    for (PlannedPass& P : planned) order_lazy_pairs(&P.gates, tables);
   std::vector<uint32_t> table_offsets;
   FlatTables flat = flatten(gates, tables, &table_offsets);
   std::vector<TileGate> all;
