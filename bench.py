@@ -572,10 +572,13 @@ def gpu_arm(args) -> None:
                          "unit": "GB/s", "frac": achieved / peaks["hbm_gbs"], "traffic": traffic,
                          "peak_source": peaks["source"],
                          "note": "achieved = 32 N bytes (one read + one write of the state) per tile pass / mean "
-                                 "tile-pass time; the tile passes are FP64-issue bound, see fp64"},
+                                 "tile-pass time; exact passes are bound by FP64 issue (see fp64), fast ones "
+                                 "by integer issue (64-bit fixed-point tiles)"},
             "fp64": {"achieved": fp64_achieved, "peak": fma_rate, "unit": "FP64 instr/s", "frac": fp64_achieved / fma_rate,
                      "peak_before": fma_rate_before, "peak_after": fma_rate_after,
-                     "note": "FP64-pipe instructions the gates need / device time of the passes; peak = DFMA issue "
+                     "note": "instructions the gates need in FP64 arithmetic / device time of the passes (part of "
+                             "them, in fast mode nearly all, run on the integer pipes instead: frac can pass 1); "
+                             "peak = DFMA issue "
                              "rate measured live on this GPU before and after the timed region "
                              "(spz_probe_fp64_fma_rate), the larger of the two"},
             "parity": parity,

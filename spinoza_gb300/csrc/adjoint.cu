@@ -212,7 +212,7 @@ __global__ void inner_re_kernel(const double* __restrict__ pr, const double* __r
 // 128 threads x 6 blocks per SM (what the tiles' shared memory allows): with the
 // products on the integer pipes 12 warps per SM (64 threads) no longer fill the
 // FP64 pipe.  21 qubits, 6 layers, the six passes: 15.2 ms with DFMA products and
-// 64 threads, 10.8 ms now.
+// 64 threads, 10.8 ms so (RZ then still on both halves).
 #ifndef SPZ_ADJ_THREADS
 #define SPZ_ADJ_THREADS 128
 #endif

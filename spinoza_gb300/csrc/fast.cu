@@ -1,8 +1,9 @@
 // Fast-mode lowering for the fused executor (opt-in, SPZ_EXEC_FAST).
 //
 // On GB300 every dense FP64 gate is bound by FP64 issue, so fast mode rewrites
-// the circuit into mathematically identical ops that need fewer FP64
-// instructions (results differ from the exact mode by rounding only):
+// the circuit into mathematically identical ops that need fewer instructions and
+// have a fixed-point form on the integer pipes (tile_fixed.cuh); results differ
+// from the exact mode by rounding only:
 //
 //   * lazy scaling: H, RX and RY are applied as the gate divided by a scalar
 //     (1/sqrt2, cos or sin of theta/2, whichever is larger in magnitude, so
