@@ -734,6 +734,13 @@ int adjoint_gradient(spz_state_t h, const spz_op* ops, size_t nops, const uint32
   const int c = std::min<int>(kTileLowBits, k);
   std::vector<PlannedPass> passes;
   for (PlannedPass& P : plan_passes(bwd, n, k, c, /*exact=*/false)) {
+    // Tiles of 2^k: a pass whose gates touch fewer qubits takes the lowest others too.
+    uint64_t L = 0;
+    for (int q : P.local) L |= 1ull << q;
+    for (int q = 0; q < (int)n && __builtin_popcountll(L) < k; ++q) L |= 1ull << q;
+    P.local.clear();
+    for (int q = 0; q < (int)n; ++q)
+      if ((L >> q) & 1) P.local.push_back(q);
     PlannedPass cur;
     cur.local = P.local;
     int slots = 0;
