@@ -1081,39 +1081,45 @@ bool lazy_pair_fits(const GateApp& a, const GateApp& b, const std::vector<PhaseT
 
 // Reorder a pass's gates (any two that commute) so that lazy ops that fit
 // together stand side by side: a partner further on moves up to its lazy op, or
-// the lazy op down to it.  (30-qubit brickwork, 20 layers: 269 pairs instead of
-// 261; few more fit, a layer's gates inside one pass being an odd number.)
+// the lazy op down to it.  A gate is paired at most once and a paired gate is
+// never moved by itself again, so every step either goes on by a gate or pairs
+// two: the work is at most kReach tests per gate.  (30-qubit brickwork, 20
+// layers: 269 pairs instead of 261; few more fit, a layer's gates inside one
+// pass being an odd number.)
 void order_lazy_pairs(std::vector<GateApp>* gates, const std::vector<PhaseTable>& tables) {
   if (!fast_pairs_enabled()) return;
   std::vector<GateApp>& g = *gates;
-  auto commute = [](const GateApp& a, const GateApp& b) {
-    return (nd_mask(a) & (nd_mask(b) | d_mask(b))) == 0 && (d_mask(a) & nd_mask(b)) == 0;
-  };
+  std::vector<char> paired(g.size(), 0);
   constexpr size_t kReach = 64;
-  for (size_t i = 0; i + 1 < g.size(); ++i) {
-    if (!lazy_uncontrolled(g[i])) continue;
-    if (lazy_pair_fits(g[i], g[i + 1], tables)) {
-      ++i;
-      continue;
+  auto move = [&](size_t from, size_t to) {  // gate `from` to position `to`, those between by one
+    auto turn = [&](auto first) {
+      if (from < to) std::rotate(first + (ptrdiff_t)from, first + (ptrdiff_t)from + 1, first + (ptrdiff_t)to + 1);
+      else std::rotate(first + (ptrdiff_t)to, first + (ptrdiff_t)from, first + (ptrdiff_t)from + 1);
+    };
+    turn(g.begin());
+    turn(paired.begin());
+  };
+  for (size_t i = 0; i + 1 < g.size();) {
+    size_t next = i + 1;
+    if (!paired[i] && lazy_uncontrolled(g[i])) {
+      const uint64_t ind = nd_mask(g[i]), id = d_mask(g[i]);
+      uint64_t nd = 0, d = 0;  // what the gates between i and j act on
+      for (size_t j = i + 1; j < g.size() && j < i + kReach; ++j) {
+        const uint64_t jnd = nd_mask(g[j]), jd = d_mask(g[j]);
+        const bool up = (jnd & (nd | d)) == 0 && (jd & nd) == 0, down = (ind & (nd | d)) == 0 && (id & nd) == 0;
+        if ((up || down) && !paired[j] && lazy_pair_fits(g[i], g[j], tables)) {
+          if (up) move(j, i + 1);
+          else move(i, j - 1);
+          const size_t at = up ? i : j - 1;
+          paired[at] = paired[at + 1] = 1;
+          next = up ? i + 2 : i;  // (down: the gate now at i has not been looked at)
+          break;
+        }
+        nd |= jnd;
+        d |= jd;
+      }
     }
-    for (size_t j = i + 2; j < g.size() && j < i + kReach; ++j) {
-      if (!lazy_pair_fits(g[i], g[j], tables)) continue;
-      bool up = true, down = true;
-      for (size_t b = i + 1; b < j; ++b) {
-        up = up && commute(g[j], g[b]);
-        down = down && commute(g[i], g[b]);
-      }
-      if (up) {
-        std::rotate(g.begin() + (ptrdiff_t)i + 1, g.begin() + (ptrdiff_t)j, g.begin() + (ptrdiff_t)j + 1);
-        ++i;
-        break;
-      }
-      if (down) {
-        std::rotate(g.begin() + (ptrdiff_t)i, g.begin() + (ptrdiff_t)i + 1, g.begin() + (ptrdiff_t)j);
-        --i;  // the gate now at i has not been looked at
-        break;
-      }
-    }
+    i = next;
   }
 }
 
