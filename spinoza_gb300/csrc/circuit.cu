@@ -838,7 +838,7 @@ FxLazy fx_lazy(int kind, double c) {
 struct FlatTables {
   std::vector<double2> entries;
   std::vector<int4> fixed;
-  bool finite = true;  // false: an angle was infinite or NaN, which fixed point cannot carry
+  bool finite = true;  // false: a coefficient is infinite or NaN, which fixed point cannot carry
   void push(std::complex<double> w, int exponent, int turn) {
     entries.push_back(make_double2(w.real(), w.imag()));
     if (!std::isfinite(w.real()) || !std::isfinite(w.imag())) {
@@ -867,8 +867,13 @@ FlatTables flatten(const std::vector<GateApp>& gates, const std::vector<PhaseTab
   for (const GateApp& g : gates)
     if (g.table >= 0 && g.kind != FK_PHASE) turn[g.table] = fx_lazy(g.kind, g.c.cs).pre;
   FlatTables f;
-  for (const GateApp& g : gates)
-    if (g.kind >= FK_LAZY_H && g.kind <= FK_LAZY_RY_B && !std::isfinite(g.c.cs)) f.finite = false;
+  // Lazy ops and the gates that stay exact (fx_exact_pair and fx_exact_diag turn
+  // their FP64 results back, which have to be finite too).
+  for (const GateApp& g : gates) {
+    const Coef& c = g.c;
+    for (double v : {c.a, c.k, c.l, c.q, c.r, c.s, c.t, c.cs, c.sn, c.nsn, c.d0re, c.d0im, c.d1re, c.d1im})
+      f.finite = f.finite && std::isfinite(v);
+  }
   for (size_t k = 0; k < tables.size(); ++k) {
     const PhaseTable& t = tables[k];
     offsets->push_back((uint32_t)f.entries.size());

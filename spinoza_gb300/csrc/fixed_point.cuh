@@ -14,7 +14,7 @@
 // that it mixes, where FP64 rounds every operation to 2^-53 of its result.  The
 // amplitudes become FP64 again, rounded to nearest, when the pass stores them.
 // Tiles with a component that is not finite or a nonzero amplitude outside
-// [2^-895, 2^881) are worked on in FP64 (fx_in_range).
+// [2^-895, 2^600) are worked on in FP64 (fx_in_range).
 //
 // Bounds.  An op's inputs have components below 2^59: a phase leaves them below
 // 2^59.5, a rotation below 2^60.5, a second one below 2^61.5; the limbs need
@@ -33,7 +33,10 @@
 namespace spz {
 
 constexpr uint32_t kFxMinHi = 0x08000000u;  // upper words of an amplitude's larger component: at least this ...
-constexpr uint32_t kFxMaxHi = 0x77000000u;  // ... and below this
+// ... and below this.  The lazy ops of a circuit grow a tile's norm by 2^401 at
+// most before the carried scale is folded in, so that an amplitude stays finite
+// where an exact gate takes it through FP64.
+constexpr uint32_t kFxMaxHi = 0x65700000u;
 constexpr int kFxZeroExp = -(1 << 28);      // exponent of a zero amplitude
 
 struct FxAmp {
