@@ -9,7 +9,6 @@
 // partials in a fixed tree.  Results are identical from run to run.
 #include <algorithm>
 #include <cmath>
-#include <cstring>
 #include <vector>
 
 #include "common.cuh"
@@ -422,22 +421,14 @@ __global__ void __launch_bounds__(kRedThreads) x_pauli_kernel(const double* __re
 //    the pair's contribution to Re<psi|P|psi>, one accumulator per term.
 // Each term's accumulators are reduced once at the end (fixed order).
 //
-// In FP64 the pass is bound by DFMA issue (16 cycles of the SM's FP64 unit per
-// warp instruction, two per pair and term), so a tile is taken to fixed point
-// when it can hold it: components as 64-bit integers below 2^58 on the exponent
-// of the tile's largest one, each as two signed limbs (v = h 2^30 + l), so that
-// a pair's part of a term is six 32 x 32-bit multiply-adds of 1.3 cycles (l * l,
-// below 2^-58 of the tile's largest probability and of either sign, is left out)
-// and a thread's sum over a tile becomes FP64 once.  A tile stays in FP64 when a
-// component is more than 2^20 below its largest (fixed point would hold fewer
-// than 38 of its bits), not finite, or the largest is not within 2^-474 ..
-// 2^476 (2 % of the tiles of a random state); a tile of zeros adds nothing.
-// 26 qubits, <X> of every qubit and the energy of an Ising chain (52 X terms, 25
-// ZZ): 7.6 ms in FP64, 5.8 ms; what is left is shared between the integer pipes
-// (42 % busy), the shared-memory pipe (54 %) and the sums' conversions (FP64 35 %).
+// DFMA issue bounds the passes, two per pair and term (26 qubits, <X> of every
+// qubit and an Ising chain's energy: 7.9 ms).  A tile as 64-bit integers on one
+// exponent took 5.8 ms, but held components 2^6 and more below the tile's largest
+// in fewer bits than FP64: a sum that is small against the largest probability
+// lost them.
 constexpr int kPtMaxTerms = 16;   // X-type terms per pass
 constexpr int kPtMaxDiag = 64;    // diagonal terms (8 chunks of 8)
-constexpr int kPtK = 12, kPtLow = 3, kPtThreads = 256;
+constexpr int kPtK = 12, kPtLow = 3, kPtThreads = 512;
 
 struct PtTerm {
   uint32_t xl;      // X-mask in local bits
@@ -460,47 +451,19 @@ struct PtArgs {
   // w(base | e) = w(base) ^ L0[e & 63] ^ L1[e >> 6] for the tile offset e.
   uint8_t lz[kPtMaxDiag / 8][2][64];
   double dconst;             // C = sum of the diagonal coefficients
-  int fixed;                 // fixed point may be used
-  const int64_t* dfix;       // dtab's layout: sums of +-c_k (no C apart), in dscale 2^-61
-  double dscale;
   int nt;
   PtTerm t[kPtMaxTerms];
   double* partials;          // (nt + 1) x gridDim.x
 };
 
-constexpr int kPfShift = 5;          // 53-bit significands to below 2^58
-constexpr uint32_t kPfSpread = 20;
-
-// The component with bits b on exponent E, rounded.  x: l, y: h.
-__device__ __forceinline__ int2 pf_from(uint64_t b, uint32_t E) {
-  const uint32_t hi = (uint32_t)(b >> 32), f = (hi >> 20) & 0x7FFu;
-  const uint64_t m = (((uint64_t)((hi & 0x000FFFFFu) | 0x00100000u) << 32) | (uint32_t)b) << (kPfShift + 1);
-  const int64_t s = (int64_t)((int32_t)hi >> 31);
-  const uint64_t u = f == 0 ? 0 : ((m >> (E - f)) + 1) >> 1;
-  const int64_t v = ((int64_t)u ^ s) - s;
-  return make_int2((int32_t)((uint32_t)v << 2) >> 2, (int32_t)((v + (1 << 29)) >> 30));
-}
-
-__device__ __forceinline__ int64_t pf_mul(int32_t a, int32_t b) { return (int64_t)a * b; }
-
-// (x + 2^(n-1)) >> n
-template <int n>
-__device__ __forceinline__ int64_t pf_round(int64_t x) {
-  return (x + (1ll << (n - 1))) >> n;
-}
-
-__global__ void __launch_bounds__(kPtThreads, 4) pauli_tile_kernel(const __grid_constant__ PtArgs A) {
+__global__ void __launch_bounds__(kPtThreads) pauli_tile_kernel(PtArgs A) {
   extern __shared__ double sm[];
   const uint32_t T = 1u << A.k;
   double* sre = sm;
   double* sim = sm + T;
-  int2* fre = reinterpret_cast<int2*>(sre);
-  int2* fim = reinterpret_cast<int2*>(sim);
   uint64_t* rowoff = reinterpret_cast<uint64_t*>(sm + 2 * T);
   double* red = sm + 2 * T + (T >> kPtLow) + 1;
-  __shared__ uint2 s_range[kPtThreads / 32];  // largest and smallest upper words
   const uint32_t cmask = (1u << A.c) - 1;
-  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   for (uint32_t r = threadIdx.x; r < (1u << A.nhigh); r += blockDim.x) {
     uint64_t off = 0;
     for (int j = 0; j < A.nhigh; ++j)
@@ -508,13 +471,9 @@ __global__ void __launch_bounds__(kPtThreads, 4) pauli_tile_kernel(const __grid_
     rowoff[r] = off;
   }
   const int nch = (A.ndiag + 7) / 8;
-  double* stab = red + 32;                                              // nch x 256 chunk tables
-  int64_t* sfix = reinterpret_cast<int64_t*>(stab + (size_t)nch * 256);
-  uint8_t* slz = reinterpret_cast<uint8_t*>(sfix + (size_t)nch * 256);  // nch x 2 x 64
-  for (int j = threadIdx.x; j < nch * 256; j += blockDim.x) {
-    stab[j] = A.dtab[j];
-    if (A.fixed) sfix[j] = A.dfix[j];
-  }
+  double* stab = red + 32;                                          // nch x 256 chunk tables
+  uint8_t* slz = reinterpret_cast<uint8_t*>(stab + (size_t)nch * 256);  // nch x 2 x 64
+  for (int j = threadIdx.x; j < nch * 256; j += blockDim.x) stab[j] = A.dtab[j];
   for (int j = threadIdx.x; j < nch * 128; j += blockDim.x) slz[j] = (&A.lz[0][0][0])[j];
   double acc[kPtMaxTerms + 1];
 #pragma unroll
@@ -522,48 +481,13 @@ __global__ void __launch_bounds__(kPtThreads, 4) pauli_tile_kernel(const __grid_
   __syncthreads();
   for (uint64_t tile = blockIdx.x; tile < A.ntiles; tile += gridDim.x) {
     const uint64_t base = deposit(tile, A.lpos, A.k);
-    uint32_t big = 0, low = ~0u;
     for (uint32_t e2 = threadIdx.x; e2 < T / 2; e2 += blockDim.x) {
       const uint32_t e = 2 * e2;
       const uint64_t gi = base | rowoff[e >> A.c] | (e & cmask);
-      const int4 r = *reinterpret_cast<const int4*>(A.re + gi), m = *reinterpret_cast<const int4*>(A.im + gi);
-      *reinterpret_cast<int4*>(sre + e) = r;
-      *reinterpret_cast<int4*>(sim + e) = m;
-      const int2 v[4] = {{r.x, r.y}, {r.z, r.w}, {m.x, m.y}, {m.z, m.w}};
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const uint32_t a = (uint32_t)v[j].y & 0x7FFFFFFFu;
-        big = max(big, a);
-        low = min(low, (a | (uint32_t)v[j].x) == 0 ? ~0u : a);
-      }
+      *reinterpret_cast<double2*>(sre + e) = *reinterpret_cast<const double2*>(A.re + gi);
+      *reinterpret_cast<double2*>(sim + e) = *reinterpret_cast<const double2*>(A.im + gi);
     }
-    big = __reduce_max_sync(0xffffffffu, big);
-    low = __reduce_min_sync(0xffffffffu, low);
-    if (lane == 0) s_range[warp] = make_uint2(big, low);
     __syncthreads();
-    const uint2 rg = s_range[lane < nwarps ? lane : 0];
-    big = __reduce_max_sync(0xffffffffu, rg.x);
-    low = __reduce_min_sync(0xffffffffu, rg.y);
-    const uint32_t E = big >> 20;
-    // the same for the whole block
-    const bool fixed = A.fixed && E >= 549u && E <= 1499u && (low >> 20) + kPfSpread >= E;
-    if (low == ~0u && A.fixed) {  // zeros, finite coefficients
-      __syncthreads();
-      continue;
-    }
-    if (fixed) {
-      for (uint32_t e2 = threadIdx.x; e2 < T / 2; e2 += blockDim.x) {  // what this thread loaded
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const uint32_t e = 2 * e2 + j;
-          fre[e] = pf_from((uint64_t)__double_as_longlong(sre[e]), E);
-          fim[e] = pf_from((uint64_t)__double_as_longlong(sim[e]), E);
-        }
-      }
-      __syncthreads();
-    }
-    // a component is v 2^(E - 1080): a sum of products over 2^60 counts 2^(2 E - 2100)
-    const double scale = __hiloint2double((int)((2 * E - 2100 + 1023) << 20), 0);
     if (A.ndiag) {
       uint32_t wb[kPtMaxDiag / 8];  // the tile base's part of each chunk index
 #pragma unroll
@@ -574,109 +498,55 @@ __global__ void __launch_bounds__(kPtThreads, 4) pauli_tile_kernel(const __grid_
           for (int j = 0; j < jn; ++j) wb[ch] |= (uint32_t)(__popcll(base & A.dz[ch * 8 + j]) & 1) << j;
         }
       }
-      if (fixed) {
-        int64_t sum = 0, cross = 0;  // at most 16 elements, |sum| and |cross| below 2^62
-        for (uint32_t e = threadIdx.x; e < T; e += blockDim.x) {
-          const uint32_t e0 = e & 63, e1 = (e >> 6) & 63;
-          int64_t d = 0;  // |d| <= 2^61, but for roundings
+      for (uint32_t e = threadIdx.x; e < T; e += blockDim.x) {
+        double d = A.dconst;
+        const uint32_t e0 = e & 63, e1 = (e >> 6) & 63;
 #pragma unroll
-          for (int ch = 0; ch < kPtMaxDiag / 8; ++ch) {
-            if (ch >= nch) break;
-            d += sfix[ch * 256 + (wb[ch] ^ slz[ch * 128 + e0] ^ slz[ch * 128 + 64 + e1])];
-          }
-          const int2 a = fre[e], b = fim[e];
-          // (re^2 + im^2) / 2^56, below 2^61
-          const int64_t p = ((pf_mul(a.y, a.y) + pf_mul(b.y, b.y)) << 4) +
-                            pf_round<25>(pf_mul(a.y, a.x) + pf_mul(b.y, b.x) +
-                                         ((pf_mul(a.x, a.x) + pf_mul(b.x, b.x)) >> 31));
-          const int32_t pl = (int32_t)(uint32_t)p, dl = (int32_t)(uint32_t)d;
-          const int32_t ph = (int32_t)(p >> 32) + (int32_t)((uint32_t)pl >> 31);
-          const int32_t dh = (int32_t)(d >> 32) + (int32_t)((uint32_t)dl >> 31);
-          sum += pf_mul(ph, dh);
-          cross += (pf_mul(ph, dl) + pf_mul(pl, dh)) >> 8;
+        for (int ch = 0; ch < kPtMaxDiag / 8; ++ch) {
+          if (ch >= nch) break;
+          const uint32_t w = wb[ch] ^ slz[ch * 128 + e0] ^ slz[ch * 128 + 64 + e1];
+          d = dadd(d, stab[ch * 256 + w]);
         }
-        sum += pf_round<24>(cross);
-        // counts dscale 2^(2 E - 2101)
-        acc[kPtMaxTerms] = dadd(dmul(dmul((double)sum, dmul(scale, 0.5)), A.dscale), acc[kPtMaxTerms]);
-      } else {
-        double sum = 0.0;
-        for (uint32_t e = threadIdx.x; e < T; e += blockDim.x) {
-          double d = A.dconst;
-          const uint32_t e0 = e & 63, e1 = (e >> 6) & 63;
-#pragma unroll
-          for (int ch = 0; ch < kPtMaxDiag / 8; ++ch) {
-            if (ch >= nch) break;
-            d = dadd(d, stab[ch * 256 + (wb[ch] ^ slz[ch * 128 + e0] ^ slz[ch * 128 + 64 + e1])]);
-          }
-          const double a = sre[e], b = sim[e];
-          sum = dfma(dfma(a, a, dmul(b, b)), d, sum);
-        }
-        acc[kPtMaxTerms] = dadd(acc[kPtMaxTerms], sum);
+        const double a = sre[e], b = sim[e];
+        acc[kPtMaxTerms] = dfma(dfma(a, a, dmul(b, b)), d, acc[kPtMaxTerms]);
       }
     }
 #pragma unroll
     for (int t = 0; t < kPtMaxTerms; ++t) {
       if (t >= A.nt) break;
-      const PtTerm& P = A.t[t];
-      const uint32_t lowmask = (1u << P.lowbit) - 1, xl = P.xl;
-      int64_t s = 0, u = 0;  // at most 8 pairs: |s| <= 2^60, |u| <= 2^62
-      if (fixed && P.simple != 0) {
-        const int2* __restrict__ fc = P.simple == 1 ? fre : fim;
-        const int2* __restrict__ fd = P.simple == 1 ? fim : fre;
-        int64_t s2 = 0, u2 = 0;
-#pragma unroll 2
-        for (uint32_t m = threadIdx.x; m < T / 2; m += blockDim.x) {
-          const uint32_t x = ((m & ~lowmask) << 1) | (m & lowmask), y = x ^ xl;
-          const int2 a = fre[x], b = fim[x], c = fc[y], d = fd[y];
-          s += pf_mul(a.y, c.y);
-          u += pf_mul(a.y, c.x);
-          u += pf_mul(a.x, c.y);
-          s2 += pf_mul(b.y, d.y);
-          u2 += pf_mul(b.y, d.x);
-          u2 += pf_mul(b.x, d.y);
-        }
-        s = P.simple == 1 ? s + s2 : s - s2;
-        u = P.simple == 1 ? u + u2 : u - u2;
-        acc[t] = dfma((double)(s + pf_round<30>(u)), scale, acc[t]);
-        continue;
-      }
+      const PtTerm P = A.t[t];
+      const uint32_t lowmask = (1u << P.lowbit) - 1;
       for (uint32_t m = threadIdx.x; m < T / 2; m += blockDim.x) {
-        const uint32_t x = ((m & ~lowmask) << 1) | (m & lowmask), y = x ^ xl;
-        // Re (even) or Im (odd) of conj(psi_x) psi_y, added, subtracted or, where
-        // the pair's two halves cancel, left out; the factor 2 is applied at the end
-        bool odd = P.simple == 2, neg = false;
-        if (P.simple == 0) {
-          const uint64_t gx = base | rowoff[x >> A.c] | (x & cmask), gy = base | rowoff[y >> A.c] | (y & cmask);
-          const int px = __popcll(gx & P.z) & 1, py = __popcll(gy & P.z) & 1, ny = P.ny & 3;
-          odd = (ny & 1) != 0;
-          if ((px != py) != odd) continue;
-          neg = odd ? (py != 0) != (ny == 1) : (px != 0) != (ny != 0);
-        }
-        if (fixed) {
-          const int2 a = fre[x], b = fim[x];
-          int2 c = fre[y], d = fim[y];
-          if (odd) {  // a d - b c
-            const int2 w = c;
-            c = d;
-            d = make_int2(-w.x, -w.y);
-          }
-          if (neg) {
-            c = make_int2(-c.x, -c.y);
-            d = make_int2(-d.x, -d.y);
-          }
-          s += pf_mul(a.y, c.y);
-          u += pf_mul(a.y, c.x);
-          u += pf_mul(a.x, c.y);
-          s += pf_mul(b.y, d.y);
-          u += pf_mul(b.y, d.x);
-          u += pf_mul(b.x, d.y);
+        const uint32_t x = ((m & ~lowmask) << 1) | (m & lowmask);
+        const uint32_t y = x ^ P.xl;
+        const double a = sre[x], b = sim[x], c = sre[y], d = sim[y];
+        if (P.simple == 1) {  // 2 Re(conj(psi_x) psi_y); the factor 2 is applied at the end
+          acc[t] = dfma(a, c, acc[t]);
+          acc[t] = dfma(b, d, acc[t]);
+        } else if (P.simple == 2) {  // 2 Im(conj(psi_x) psi_y)
+          acc[t] = dfma(a, d, acc[t]);
+          acc[t] = dfma(dneg(b), c, acc[t]);
         } else {
-          const double a = sre[x], b = sim[x], c = odd ? sim[y] : sre[y], d = odd ? sre[y] : sim[y];
-          acc[t] = dfma(neg ? dneg(a) : a, c, acc[t]);
-          acc[t] = dfma(neg != odd ? dneg(b) : b, d, acc[t]);
+          const uint64_t gx = base | rowoff[x >> A.c] | (x & cmask);
+          const uint64_t gy = base | rowoff[y >> A.c] | (y & cmask);
+          const int sx = (__popcll(gx & P.z) & 1) ? -1 : 1;
+          const int sy = (__popcll(gy & P.z) & 1) ? -1 : 1;
+          const int ny = P.ny & 3;
+          const double wre = dfma(a, c, dmul(b, d)), wim = dfma(a, d, dmul(dneg(b), c));
+          int f;
+          double v;
+          if ((ny & 1) == 0) {
+            f = (sx + sy) * (ny == 0 ? 1 : -1);
+            v = wre;
+          } else {
+            f = (sy - sx) * (ny == 1 ? -1 : 1);
+            v = wim;
+          }
+          // half of f * v (f is -2, 0 or 2): the factor 2 is applied at the end
+          if (f > 0) acc[t] = dadd(acc[t], v);
+          else if (f < 0) acc[t] = dsub(acc[t], v);
         }
       }
-      if (fixed) acc[t] = dfma((double)(s + pf_round<30>(u)), scale, acc[t]);
     }
     __syncthreads();
   }
@@ -687,10 +557,11 @@ __global__ void __launch_bounds__(kPtThreads, 4) pauli_tile_kernel(const __grid_
     const int row = s == kPtMaxTerms ? A.nt : s;
     double v = acc[s];
     for (int off = 16; off > 0; off >>= 1) v = dadd(v, __shfl_down_sync(0xffffffffu, v, off));
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (lane == 0) red[warp] = v;
     __syncthreads();
     if (warp == 0) {
-      double r = lane < nwarps ? red[lane] : 0.0;
+      double r = lane < (int)(blockDim.x >> 5) ? red[lane] : 0.0;
       for (int off = 16; off > 0; off >>= 1) r = dadd(r, __shfl_down_sync(0xffffffffu, r, off));
       if (lane == 0) A.partials[(size_t)row * gridDim.x + blockIdx.x] = r;
     }
@@ -705,61 +576,43 @@ static int pauli_tiles(spz_state_t h, const spz_pauli_term* terms, size_t nterms
                        double* per_term = nullptr) {
   *done = false;
   const uint32_t n = h->n;
-  const int c = std::min<int>(kPtLow, (int)n);
+  const int k = std::min<int>((int)n, kPtK);
+  const int c = std::min<int>(kPtLow, k);
   std::vector<size_t> diag, xt;
   for (size_t i = 0; i < nterms; ++i) (terms[i].x_mask ? xt : diag).push_back(i);
   if (diag.size() > (size_t)kPtMaxDiag) return SPZ_OK;
   for (size_t i : xt)
-    if (__builtin_popcountll(terms[i].x_mask) > std::min<int>((int)n, kPtK) - c) return SPZ_OK;
+    if (__builtin_popcountll(terms[i].x_mask) > k - c) return SPZ_OK;
   // passes: greedy local sets covering the X-masks
   struct Pass { std::vector<int> local; std::vector<size_t> terms; bool diag; };
-  auto cover = [&](int k) {
-    std::vector<Pass> passes;
-    std::vector<int> done_t(xt.size(), 0);
-    size_t left = xt.size();
-    bool first = true;
-    while (left > 0 || first) {
-      uint64_t L = (1ull << c) - 1;
-      int nl = c;
-      Pass P;
-      P.diag = first && !diag.empty();
-      for (size_t j = 0; j < xt.size() && (int)P.terms.size() < kPtMaxTerms; ++j) {
-        if (done_t[j]) continue;
-        const uint64_t need = terms[xt[j]].x_mask & ~L;
-        const int add = __builtin_popcountll(need);
-        if (nl + add <= k) {
-          L |= need;
-          nl += add;
-          P.terms.push_back(xt[j]);
-          done_t[j] = 1;
-          left--;
-        }
-      }
-      for (int q = 0; q < (int)n && nl < k; ++q)
-        if (!((L >> q) & 1)) { L |= 1ull << q; nl++; }
-      for (int q = 0; q < (int)n; ++q)
-        if ((L >> q) & 1) P.local.push_back(q);
-      first = false;
-      if (P.diag || !P.terms.empty()) passes.push_back(std::move(P));
-      if (left == 0) break;
-    }
-    return passes;
-  };
-  // Tiles of 2^11 amplitudes: four blocks of 256 threads in an SM, whose loads and
-  // sums overlap (26 qubits, 26 X terms and the chain: 2.9 ms; tiles of 2^12 with
-  // two blocks of 512 threads 3.0 ms); of 2^12 where those need fewer passes (28
-  // qubits, 3 passes instead of 4: 22.5 ms for twice the 28 terms, 25.4 with 2^11).
-  int k = std::min<int>((int)n, kPtK - 1);
-  bool narrow = true;
-  for (size_t i : xt) narrow = narrow && __builtin_popcountll(terms[i].x_mask) <= k - c;
   std::vector<Pass> passes;
-  if (narrow) passes = cover(k);
-  if (!narrow || (passes.size() > 1 && (int)n >= kPtK)) {
-    std::vector<Pass> wide = cover(std::min<int>((int)n, kPtK));
-    if (!narrow || wide.size() < passes.size()) {
-      passes = std::move(wide);
-      k = std::min<int>((int)n, kPtK);
+  std::vector<int> done_t(xt.size(), 0);
+  size_t left = xt.size();
+  bool first = true;
+  while (left > 0 || first) {
+    uint64_t L = (1ull << c) - 1;
+    int nl = c;
+    Pass P;
+    P.diag = first && !diag.empty();
+    for (size_t j = 0; j < xt.size() && (int)P.terms.size() < kPtMaxTerms; ++j) {
+      if (done_t[j]) continue;
+      const uint64_t need = terms[xt[j]].x_mask & ~L;
+      const int add = __builtin_popcountll(need);
+      if (nl + add <= k) {
+        L |= need;
+        nl += add;
+        P.terms.push_back(xt[j]);
+        done_t[j] = 1;
+        left--;
+      }
     }
+    for (int q = 0; q < (int)n && nl < k; ++q)
+      if (!((L >> q) & 1)) { L |= 1ull << q; nl++; }
+    for (int q = 0; q < (int)n; ++q)
+      if ((L >> q) & 1) P.local.push_back(q);
+    first = false;
+    if (P.diag || !P.terms.empty()) passes.push_back(std::move(P));
+    if (left == 0) break;
   }
   // diagonal tables
   const size_t nd = diag.size();
@@ -774,27 +627,7 @@ static int pauli_tiles(spz_state_t h, const spz_pauli_term* terms, size_t nterms
         if ((v >> b) & 1) s += -2.0 * terms[diag[ch * 8 + b]].coeff;
       tab[ch * 256 + v] = s;
     }
-  double dscale = 0.0;
-  for (size_t j = 0; j < nd; ++j) dscale += std::fabs(terms[diag[j]].coeff);
-  const bool fixed = nd == 0 || (dscale > 1e-280 && dscale < 1e280);
-  if (fixed && nd) {
-    const size_t at = tab.size();
-    int e;
-    std::frexp(dscale, &e);
-    dscale = std::ldexp(1.0, e);  // a power of two: exact both ways
-    const double up = std::ldexp(1.0, 61 - e);
-    tab.resize(2 * at);
-    for (size_t ch = 0; ch < nchunks; ++ch)
-      for (int v = 0; v < 256; ++v) {
-        int64_t s = 0;
-        for (int b = 0; b < 8 && ch * 8 + b < nd; ++b) {
-          const int64_t c = (int64_t)std::llrint(terms[diag[ch * 8 + b]].coeff * up);
-          s += ((v >> b) & 1) ? -c : c;
-        }
-        std::memcpy(&tab[at + ch * 256 + v], &s, sizeof s);
-      }
-  }
-  const int blocks = (int)std::min<uint64_t>(1ull << (n - k), (uint64_t)kNumSMs * (k == kPtK ? 3 : 4));
+  const int blocks = (int)std::min<uint64_t>(1ull << (n - k), (uint64_t)kNumSMs * 3);
   const size_t slots_per_pass = (size_t)(kPtMaxTerms + 1) * blocks;
   const size_t nres = passes.size() * (kPtMaxTerms + 1);
   void* scratch;
@@ -811,8 +644,7 @@ static int pauli_tiles(spz_state_t h, const spz_pauli_term* terms, size_t nterms
     std::lock_guard<std::mutex> lock(attr_mu);
     if (!attr[h->device]) {
       SPZ_CUDA(cudaFuncSetAttribute(pauli_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)((2 << kPtK) + (1 << (kPtK - kPtLow)) + 64 +
-                                          (kPtMaxDiag / 8) * (2 * 256 + 16)) * 8));
+                                    (int)((2 << kPtK) + (1 << (kPtK - kPtLow)) + 64 + (kPtMaxDiag / 8) * (256 + 16)) * 8));
       attr[h->device] = true;
     }
   }
@@ -834,8 +666,6 @@ static int pauli_tiles(spz_state_t h, const spz_pauli_term* terms, size_t nterms
       for (size_t j = 0; j < nd; ++j) A.dz[j] = terms[diag[j]].z_mask;
       A.dtab = dtab;
       A.dconst = dconst;
-      A.dfix = (const int64_t*)(dtab + tab.size() / 2);
-      A.dscale = dscale;
       // column of tile-offset bit b in chunk ch: the chunk's terms whose Z-mask
       // holds the local qubit lpos[b]
       for (int ch = 0; ch < (int)((nd + 7) / 8); ++ch) {
@@ -867,11 +697,10 @@ static int pauli_tiles(spz_state_t h, const spz_pauli_term* terms, size_t nterms
       pt.ny = __builtin_popcountll(tm.x_mask & tm.z_mask);
       pt.simple = tm.z_mask == 0 ? 1 : (tm.z_mask == tm.x_mask && pt.ny == 1 ? 2 : 0);
     }
-    A.fixed = fixed;
     A.partials = dpart + p * slots_per_pass;
     const uint32_t T = 1u << A.k;
     const size_t nch = P.diag ? (nd + 7) / 8 : 0;
-    const size_t smem = (2 * T + (T >> kPtLow) + 1 + 32 + nch * 2 * 256 + nch * 16) * sizeof(double);
+    const size_t smem = (2 * T + (T >> kPtLow) + 1 + 32 + nch * 256 + nch * 16) * sizeof(double);
     const int threads = (int)std::min<uint32_t>(kPtThreads, std::max<uint32_t>(32, T / 2));
     const int nb = (int)std::min<uint64_t>(A.ntiles, (uint64_t)blocks);
     pauli_tile_kernel<<<nb, threads, smem, h->stream>>>(A);
