@@ -378,8 +378,8 @@ int spz_sample(spz_state_t h, const double* u, size_t nshots, uint64_t* out);
  * goes to grad[j].  On return the handle holds psi(theta), *energy = E, grad[j]
  * = dE/dtheta_j.  Needs two extra state vectors of device memory.  flags:
  * SPZ_EXEC_DEFAULT, or SPZ_EXEC_FAST (fast-mode forward, and a backward sweep
- * with lazily scaled H / RX / RY inverses: about half the FP64 work, equal to the
- * exact gradients up to rounding).
+ * with lazily scaled H / RX / RY inverses and RZ inverses as P: about half the
+ * FP64 work, equal to the exact gradients up to rounding).
  * No reference counterpart (new form built on the gate path). */
 int spz_adjoint_gradient(spz_state_t h, const spz_op* ops, size_t nops,
                          const uint32_t* param_index, size_t nparams,

@@ -1033,10 +1033,8 @@ int build_batch(spz_batch_t b, const spz_batch_instance* inst, size_t ninst, con
     std::vector<GateApp> bwd;
     for (size_t j = applied.size(); j-- > 0;) {
       GateApp inv;
-      spz_gate back = inverse_of(fwd_gate[applied[j].src]);
-      // An uncontrolled RZ goes back as P, gradient and all: see the fused adjoint sweep.
-      if (back.kind == SPZ_GATE_RZ && (applied[j].ones | applied[j].zeros) == 0) back.kind = SPZ_GATE_P;
-      int rc = make_gate_app(n, back, applied[j].target, applied[j].ones, applied[j].zeros, &inv);
+      int rc = make_gate_app(n, inverse_of(fwd_gate[applied[j].src]), applied[j].target, applied[j].ones,
+                             applied[j].zeros, &inv);
       if (rc) return rc;
       inv.src = applied[j].src;
       bwd.push_back(inv);
