@@ -31,7 +31,7 @@ class Gate:
         else:
             p = [float(v) for v in params] + [0.0] * (3 - len(params))
             self.params = tuple(p[:3])
-        if qubits:
+        if len(qubits):
             q = [int(v) for v in qubits] + [0] * (2 - len(qubits))
             self.qubits = tuple(q[:2])
         else:
