@@ -312,9 +312,9 @@ __device__ __forceinline__ void run_elementwise(const TileGate& g, const double2
     if ((e[u] & g.e_mask) != g.l_ones) continue;
     const bool one = gone >= 0 ? gone != 0 : (e[u] & g.tbit) != 0;
     switch (g.kind) {
-      case SPZ_GATE_Z: DiagGate<SPZ_GATE_Z>(g.c)(one, xr[u], xi[u]); break;
-      case SPZ_GATE_P: DiagGate<SPZ_GATE_P>(g.c)(one, xr[u], xi[u]); break;
-      default: DiagGate<SPZ_GATE_RZ>(g.c)(one, xr[u], xi[u]); break;
+      case SPZ_GATE_Z: DiagGate<SPZ_GATE_Z>(g.d)(one, xr[u], xi[u]); break;
+      case SPZ_GATE_P: DiagGate<SPZ_GATE_P>(g.d)(one, xr[u], xi[u]); break;
+      default: DiagGate<SPZ_GATE_RZ>(g.d)(one, xr[u], xi[u]); break;
     }
   }
 }

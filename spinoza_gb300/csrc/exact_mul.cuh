@@ -40,7 +40,7 @@ struct MulRange {
 SPZ_HD MulRange mul_range_all() { return MulRange{0x00100000u, 0x7FE00000u}; }
 
 // Prepare the coefficient with bits `c` and narrow r by it (to nothing when c
-// is zero, subnormal, infinite or NaN).
+// is zero, subnormal, 2^1023 or more, infinite or NaN).
 SPZ_HD MulCoef mul_prepare(uint64_t c, MulRange& r) {
   const uint32_t hi = (uint32_t)(c >> 32), lo = (uint32_t)c;
   const uint32_t ec = (hi >> 20) & 0x7FFu;
@@ -50,6 +50,8 @@ SPZ_HD MulCoef mul_prepare(uint64_t c, MulRange& r) {
   m.cl = lo << 10;
   // upper word of the product = significand (bit 20 set) + (y's sign and
   // exponent) + kexp - (s << 20), s = 1 or 2: the normalising shift
+  // (bits 31 and 30 of the exponent's part agree, so that where kexp's differ the
+  // coefficient is negative)
   m.kexp = ((ec - 1023u + 1u) << 20) + (hi & 0x80000000u);
   // exponents e_y with 1 <= e_y <= 2046 and 2 <= e_y + ec - 1023 <= 2044
   const int shift = (int)ec - 1023;
@@ -59,7 +61,7 @@ SPZ_HD MulCoef mul_prepare(uint64_t c, MulRange& r) {
   const int ra = (int)(r.lo >> 20), rb = ra + (int)(r.span >> 20) - 1;
   if (a < ra) a = ra;
   if (b > rb) b = rb;
-  if (ec == 0u || ec == 0x7FFu || b < a) {
+  if (ec == 0u || ec >= 0x7FEu || b < a) {
     r.lo = 0u;
     r.span = 0u;
   } else {
@@ -124,6 +126,29 @@ SPZ_HD uint64_t mul_int(uint64_t y, const MulCoef& c) {
   const uint64_t up = ((uint64_t)w + half) >> 32;
   return (((uint64_t)mh << 32) | ml) + up + ((uint64_t)e << 32);
 #endif
+}
+
+// The same with zeros taken too: for gates with integer instructions to spare
+// (diagonal ones), so that real-valued and part-empty states stay on this path.
+SPZ_HD bool mul_zero(uint64_t y) {
+#ifdef __CUDA_ARCH__
+  uint32_t m;  // (upper word & 0x7FFFFFFF) | lower word; in asm, or the compiler makes it an FP64 comparison
+  asm("lop3.b32 %0, %1, 0x7FFFFFFF, %2, 0xEA;" : "=r"(m) : "r"((uint32_t)(y >> 32)), "r"((uint32_t)y));
+  return m == 0u;
+#else
+  return (y << 1) == 0u;
+#endif
+}
+SPZ_HD bool mul_ok_or_zero(uint64_t y, const MulRange& r) { return mul_ok(y, r) | (mul_zero(y) & (r.span != 0u)); }
+SPZ_HD uint64_t mul_int_or_zero(uint64_t y, const MulCoef& c) {
+  const uint64_t p = mul_int(y, c);
+  const uint32_t sign = ((uint32_t)(y >> 32) ^ c.kexp ^ (c.kexp << 1)) & 0x80000000u;  // the coefficient's: see mul_prepare
+  return mul_zero(y) ? (uint64_t)sign << 32 : p;
+}
+// The coefficient with its sign flipped when `flip`.
+SPZ_HD MulCoef mul_flip(MulCoef c, bool flip) {
+  c.kexp ^= flip ? 0x80000000u : 0u;
+  return c;
 }
 
 // |y| * |y| rounded, as bits, for sqr_ok(y): mul_int with the coefficient made

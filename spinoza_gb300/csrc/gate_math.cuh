@@ -56,16 +56,34 @@ __device__ __forceinline__ void fast_pair_kind(int kind, double t, double& a, do
 // instead of 12 for RX / RY, 10 instead of 14 for U, 4 instead of 8 for RZ.
 // All eight products of a rotation on the integer pipes measured best (27
 // qubits, H + RX + RZ + U + CX + 3-control X on every target: 159.1 ms with
-// DFMA products, 109.7 with six of a rotation's eight moved, 107.5 with eight;
-// 26-qubit exact brickwork 226.4 -> 177.5 ms).
+// DFMA products, 109.7 with six of a rotation's eight moved, 107.5 with eight,
+// 100.8 with RZ's signs on the integer pipe; 26-qubit exact brickwork 226.4 ->
+// 177.5 ms).
 __device__ __forceinline__ double imul(double y, const MulCoef& c) {
   return __longlong_as_double((long long)mul_int(dbits(y), c));
 }
 
+__device__ __forceinline__ double imul_or_zero(double y, const MulCoef& c) {
+  return __longlong_as_double((long long)mul_int_or_zero(dbits(y), c));
+}
+
+// x with its sign flipped when `flip`, on the integer pipe (a negation that no FP64
+// instruction takes in as an operand's sign is an FP64 instruction itself).
+__device__ __forceinline__ double flip_sign(double x, bool flip) {
+  return __hiloint2double(__double2hiint(x) ^ (flip ? (int)0x80000000 : 0), __double2loint(x));
+}
+
+// Whether p holds in every lane that is here.  The two ways of a gate are chosen
+// by the warp, not by the lane: a warp with zeros in some lanes would otherwise
+// go both ways, one after the other, and cost more than DFMA products alone (25
+// qubits, real-valued state with a qubit in |0>: RY 657 us by lane, 403 by warp; H
+// 404 and 276).
+__device__ __forceinline__ bool warp_all(bool p) { return __all_sync(__activemask(), p) != 0; }
+
 // One gate on one pair, its coefficients prepared once (before a kernel's
 // loop).  Products by a coefficient come from the integer pipes when every
-// amplitude of the pair is in the prepared range, from dmul() otherwise; both
-// give the reference's bits.
+// amplitude of the warp's pairs is in the prepared range, from dmul() otherwise;
+// both give the reference's bits.
 template <int KIND>
 struct PairGate {
   MulRange range = mul_range_all();
@@ -94,7 +112,7 @@ struct PairGate {
   __device__ __forceinline__ void operator()(double& a, double& b, double& c, double& d) const {
     if constexpr (KIND == SPZ_GATE_H) {  // h_apply_strat2, gates.rs:547-562
       double a1, b1, c1, d1;
-      if (ok(a) && ok(b) && ok(c) && ok(d)) {
+      if (warp_all(ok(a) & ok(b) & ok(c) & ok(d))) {
         a1 = imul(a, m0); b1 = imul(b, m0); c1 = imul(c, m0); d1 = imul(d, m0);
       } else {
         a1 = dmul(kSqrtOneHalf, a); b1 = dmul(kSqrtOneHalf, b);
@@ -112,7 +130,7 @@ struct PairGate {
       a = na; b = nb; c = nc; d = nd;
     } else if constexpr (KIND == SPZ_GATE_RX) {  // rx_apply_target, gates.rs:713-725
       double ac, bc, cc, dc, an, bn, cn, dn;  // times cos, times neg_sin
-      if (ok(a) && ok(b) && ok(c) && ok(d)) {
+      if (warp_all(ok(a) & ok(b) & ok(c) & ok(d))) {
         ac = imul(a, m0); an = imul(a, m1); bc = imul(b, m0); bn = imul(b, m1);
         cc = imul(c, m0); cn = imul(c, m1); dc = imul(d, m0); dn = imul(d, m1);
       } else {
@@ -125,7 +143,7 @@ struct PairGate {
       d = dadd(dc, an);
     } else if constexpr (KIND == SPZ_GATE_RY) {  // ry_apply_strategy2, gates.rs:1116-1119
       double ac, bc, cc, dc, as, bs, cs, ds;  // times cos, times sin
-      if (ok(a) && ok(b) && ok(c) && ok(d)) {
+      if (warp_all(ok(a) & ok(b) & ok(c) & ok(d))) {
         ac = imul(a, m0); as = imul(a, m1); bc = imul(b, m0); bs = imul(b, m1);
         cc = imul(c, m0); cs = imul(c, m1); dc = imul(d, m0); ds = imul(d, m1);
       } else {
@@ -139,7 +157,7 @@ struct PairGate {
     } else if constexpr (KIND == SPZ_GATE_U) {  // u_apply_target, gates.rs:1256-1259
       const double p = a, q = b, m = c, n = d;
       double ln, lm, tn, tm;  // -l n, l m, -t n, t m
-      if (ok(m) && ok(n)) {
+      if (warp_all(ok(m) & ok(n))) {
         ln = imul(n, m0); lm = imul(m, m1); tn = imul(n, m2); tm = imul(m, m3);
       } else {
         ln = dmul(dneg(g.l), n); lm = dmul(g.l, m); tn = dmul(dneg(g.t), n); tm = dmul(g.t, m);
@@ -156,7 +174,11 @@ struct PairGate {
 
 // Diagonal gates on one amplitude; `one` is the amplitude's target bit.  RZ's
 // entries are (re, im) = (cos, -sin) on 0 and (cos, sin) on 1.
-template <int KIND>
+// ZEROS: amplitudes that are zero stay on the integer path (the per-gate kernels,
+// which HBM bounds; 25 qubits, real-valued state: RZ 366 us without, 178 with, P
+// 147 and 98).  In tile passes, where the integer pipes are the busier ones, the
+// tests cost more than they give (20-qubit QFT 632 us without, 674 with).
+template <int KIND, bool ZEROS = false>
 struct DiagGate : DiagCoef {
   __device__ __forceinline__ explicit DiagGate(const DiagCoef& d) : DiagCoef(d) {}
   __device__ __forceinline__ explicit DiagGate(const Coef& c) : DiagCoef{} {
@@ -166,26 +188,52 @@ struct DiagGate : DiagCoef {
     }
   }
 
-  __device__ __forceinline__ void operator()(bool one, double& re, double& im) const {
+  // Whether the amplitude's products may come from the integer pipes.
+  __device__ __forceinline__ bool fits(double re, double im) const {
+    const auto ok = [this](double y) { return ZEROS ? mul_ok_or_zero(dbits(y), range) : mul_ok(dbits(y), range); };
+    if constexpr (KIND == SPZ_GATE_P) return ok(re) & ok(im);
+    else if constexpr (KIND == SPZ_GATE_RZ) return ok(im);
+    else return true;
+  }
+
+  template <bool INT>
+  __device__ __forceinline__ void apply(bool one, double& re, double& im) const {
     if constexpr (KIND == SPZ_GATE_Z) {  // z_proc_chunk, gates.rs:1054-1056
       if (one) { re = dneg(re); im = dneg(im); }
     } else if constexpr (KIND == SPZ_GATE_P) {  // p_proc_chunk, gates.rs:837-838
       if (one) {
         const double zr = re, zi = im;
-        const bool ok = mul_ok(dbits(zr), range) && mul_ok(dbits(zi), range);
-        double is, rs;  // im * sin, re * sin
-        if (ok) { is = imul(zi, mim); rs = imul(zr, mim); }
-        else { is = dmul(zi, im1); rs = dmul(zr, im1); }
-        re = dfma(zr, re1, dneg(is));
+        double is, rs;  // -im * sin, re * sin
+        if constexpr (!INT) { is = dmul(dneg(zi), im1); rs = dmul(zr, im1); }
+        else if constexpr (ZEROS) { is = imul_or_zero(zi, mul_flip(mim, true)); rs = imul_or_zero(zr, mim); }
+        else { is = dneg(imul(zi, mim)); rs = imul(zr, mim); }
+        re = dfma(zr, re1, is);
         im = dfma(zi, re1, rs);
       }
     } else if constexpr (KIND == SPZ_GATE_RZ) {  // rz_apply_strategy1, gates.rs:939-946
-      const double cr = re, ci = im, s = one ? im1 : dneg(im1);
-      double is, ic;  // im * |entry's sign| sin, im * cos
-      if (mul_ok(dbits(ci), range)) { is = imul(ci, mim); ic = imul(ci, mre); }
-      else { is = dmul(ci, im1); ic = dmul(ci, re1); }
-      re = dfma(cr, re1, one ? dneg(is) : is);
+      const double cr = re, ci = im, s = flip_sign(im1, !one);
+      double is, ic;  // -im * the entry's sin, im * cos
+      if constexpr (!INT) { is = dmul(dneg(ci), s); ic = dmul(ci, re1); }
+      else if constexpr (ZEROS) { is = imul_or_zero(ci, mul_flip(mim, one)); ic = imul_or_zero(ci, mre); }
+      else { is = flip_sign(imul(ci, mim), one); ic = imul(ci, mre); }
+      re = dfma(cr, re1, is);
       im = dfma(cr, s, ic);
+    }
+  }
+
+  __device__ __forceinline__ void operator()(bool one, double& re, double& im) const {
+    if (warp_all(fits(re, im))) apply<true>(one, re, im);
+    else apply<false>(one, re, im);
+  }
+
+  // Two amplitudes of a thread, their instructions side by side.
+  __device__ __forceinline__ void operator()(bool one0, double& re0, double& im0, bool one1, double& re1, double& im1) const {
+    if (warp_all(fits(re0, im0) & fits(re1, im1))) {
+      apply<true>(one0, re0, im0);
+      apply<true>(one1, re1, im1);
+    } else {
+      apply<false>(one0, re0, im0);
+      apply<false>(one1, re1, im1);
     }
   }
 };

@@ -225,14 +225,13 @@ __global__ void __launch_bounds__(kThreads) pair_kernel_s(PairArgs A) {
 // own target bit picks the diagonal entry.
 template <int KIND>
 __global__ void __launch_bounds__(kThreads) diag_kernel_v2(PairArgs A) {
-  const DiagGate<KIND> op(A.c);
+  const DiagGate<KIND, true> op(A.c);
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < A.nwork; w += stride) {
     const uint64_t e = deposit(2 * w, A.pos, A.npos) | A.ones;
     double2 r = *reinterpret_cast<const double2*>(A.re + e);
     double2 i = *reinterpret_cast<const double2*>(A.im + e);
-    op((e & A.tbit) != 0, r.x, i.x);
-    op(((e + 1) & A.tbit) != 0, r.y, i.y);
+    op((e & A.tbit) != 0, r.x, i.x, ((e + 1) & A.tbit) != 0, r.y, i.y);
     *reinterpret_cast<double2*>(A.re + e) = r;
     *reinterpret_cast<double2*>(A.im + e) = i;
   }
@@ -240,7 +239,7 @@ __global__ void __launch_bounds__(kThreads) diag_kernel_v2(PairArgs A) {
 
 template <int KIND>
 __global__ void __launch_bounds__(kThreads) diag_kernel_s(PairArgs A) {
-  const DiagGate<KIND> op(A.c);
+  const DiagGate<KIND, true> op(A.c);
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < A.nwork; w += stride) {
     const uint64_t e = deposit(w, A.pos, A.npos) | A.ones;
