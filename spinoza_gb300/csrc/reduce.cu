@@ -1164,8 +1164,16 @@ int spz_xyz_expectation_value(spz_state_t h, char observable, const uint32_t* ta
   }
   for (uint32_t i = 0; i < ntargets; ++i)
     if (targets[i] >= h->n) return fail(SPZ_ERR_INVALID_ARGUMENT, "target qubit out of range");
-  if (ntargets == 1) return reduce_scalar(h, mode, (int)targets[0], out);
-  return ntargets ? xyz_multi(h, mode, targets, ntargets, out) : SPZ_OK;
+  // One target, or <Z> of two, takes less time by the pair reductions: a read of
+  // the state each, against four launches (20 qubits, <Z> of two 60 us against 84,
+  // of three 92 against 84) and, up to 24 qubits, more arithmetic (24 qubits 246 and
+  // 261 us; 26 qubits 798 and 747).
+  const bool one_by_one =
+      ntargets == 1 || (mode == RED_Z && ntargets == 2 && h->n > (uint32_t)kSmallMultiQubits && h->n <= 24);
+  if (!one_by_one) return ntargets ? xyz_multi(h, mode, targets, ntargets, out) : SPZ_OK;
+  for (uint32_t i = 0; i < ntargets; ++i)
+    if (int rc = reduce_scalar(h, mode, (int)targets[i], &out[i])) return rc;
+  return SPZ_OK;
 }
 
 int spz_pauli_expectation(spz_state_t h, const spz_pauli_term* terms, size_t nterms, double* out) {
