@@ -516,36 +516,30 @@ __global__ void __launch_bounds__(kPtThreads) pauli_tile_kernel(PtArgs A) {
       if (t >= A.nt) break;
       const PtTerm P = A.t[t];
       const uint32_t lowmask = (1u << P.lowbit) - 1;
-      for (uint32_t m = threadIdx.x; m < T / 2; m += blockDim.x) {
-        const uint32_t x = ((m & ~lowmask) << 1) | (m & lowmask);
-        const uint32_t y = x ^ P.xl;
-        const double a = sre[x], b = sim[x], c = sre[y], d = sim[y];
-        if (P.simple == 1) {  // 2 Re(conj(psi_x) psi_y); the factor 2 is applied at the end
+      // Re (even) or Im (odd) of conj(psi_x) psi_y; the factor 2 is applied at the end
+      if (P.simple != 0) {
+        const bool odd = P.simple == 2;
+        const double *sc = odd ? sim : sre, *sd = odd ? sre : sim;
+        for (uint32_t m = threadIdx.x; m < T / 2; m += blockDim.x) {
+          const uint32_t x = ((m & ~lowmask) << 1) | (m & lowmask), y = x ^ P.xl;
+          const double a = sre[x], b = sim[x], c = sc[y], d = sd[y];
           acc[t] = dfma(a, c, acc[t]);
-          acc[t] = dfma(b, d, acc[t]);
-        } else if (P.simple == 2) {  // 2 Im(conj(psi_x) psi_y)
-          acc[t] = dfma(a, d, acc[t]);
-          acc[t] = dfma(dneg(b), c, acc[t]);
-        } else {
-          const uint64_t gx = base | rowoff[x >> A.c] | (x & cmask);
-          const uint64_t gy = base | rowoff[y >> A.c] | (y & cmask);
-          const int sx = (__popcll(gx & P.z) & 1) ? -1 : 1;
-          const int sy = (__popcll(gy & P.z) & 1) ? -1 : 1;
-          const int ny = P.ny & 3;
-          const double wre = dfma(a, c, dmul(b, d)), wim = dfma(a, d, dmul(dneg(b), c));
-          int f;
-          double v;
-          if ((ny & 1) == 0) {
-            f = (sx + sy) * (ny == 0 ? 1 : -1);
-            v = wre;
-          } else {
-            f = (sy - sx) * (ny == 1 ? -1 : 1);
-            v = wim;
-          }
-          // half of f * v (f is -2, 0 or 2): the factor 2 is applied at the end
-          if (f > 0) acc[t] = dadd(acc[t], v);
-          else if (f < 0) acc[t] = dsub(acc[t], v);
+          acc[t] = odd ? dfma(dneg(b), d, acc[t]) : dfma(b, d, acc[t]);
         }
+        continue;
+      }
+      // with Z factors: added, subtracted or, where the pair's two halves cancel, left out
+      const int ny = P.ny & 3;
+      const bool odd = (ny & 1) != 0;
+      for (uint32_t m = threadIdx.x; m < T / 2; m += blockDim.x) {
+        const uint32_t x = ((m & ~lowmask) << 1) | (m & lowmask), y = x ^ P.xl;
+        const uint64_t gx = base | rowoff[x >> A.c] | (x & cmask), gy = base | rowoff[y >> A.c] | (y & cmask);
+        const int px = __popcll(gx & P.z) & 1, py = __popcll(gy & P.z) & 1;
+        if ((px != py) != odd) continue;
+        const bool neg = odd ? (py != 0) != (ny == 1) : (px != 0) != (ny != 0);
+        const double a = sre[x], b = sim[x], c = odd ? sim[y] : sre[y], d = odd ? sre[y] : sim[y];
+        acc[t] = neg ? dfma(dneg(a), c, acc[t]) : dfma(a, c, acc[t]);
+        acc[t] = neg != odd ? dfma(dneg(b), d, acc[t]) : dfma(b, d, acc[t]);
       }
     }
     __syncthreads();
