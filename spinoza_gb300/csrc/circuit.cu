@@ -427,15 +427,27 @@ __device__ __forceinline__ uint32_t fx_pass_gates(const PassArgs& A, uint64_t ba
     const TileGate& g = A.gates[gi];
     if constexpr (SHFL) {
       if (g.run_end > gi) {
-        for (uint32_t e = threadIdx.x; e < T; e += blockDim.x) {  // whole rows: T and blockDim are multiples of 32
-          FxAmp x = S.load(e);
+        constexpr int R = kRunRows;
+        // (T and blockDim are multiples of 32: a warp's rows are whole, and inside the
+        // tile or not for all its lanes; a row past the end repeats the first)
+        for (uint32_t e0 = threadIdx.x; e0 < T; e0 += R * blockDim.x) {
+          uint32_t e[R];
+          FxAmp row[R];
+#pragma unroll
+          for (int u = 0; u < R; ++u) {
+            const uint32_t at = e0 + u * blockDim.x;
+            e[u] = at < T ? at : e0;
+            row[u] = S.load(e[u]);
+          }
           for (int ri = gi; ri < g.run_end; ++ri) {
             const TileGate& h = A.gates[ri];
             if ((base & h.g_ones) != h.g_ones || (base & h.g_zeros) != 0) continue;
             if (h.cond >= 0 && A.outcomes[h.cond] == 0) continue;
-            fx_run_gate(h, A.fxtables, base, e, x);
+            fx_run_gate<R>(h, A.fxtables, base, e, row);
           }
-          S.store(e, x);
+#pragma unroll
+          for (int u = 0; u < R; ++u)
+            if (u == 0 || e[u] != e0) S.store(e[u], row[u]);
         }
         gi = g.run_end - 1;
         __syncthreads();
