@@ -219,7 +219,9 @@ typedef struct spz_tracker {
 #define SPZ_EXEC_TIME_PASSES 4u  /* time every pass with CUDA events (synchronises once)  */
 #define SPZ_EXEC_FAST 8u         /* fused, with arithmetic rewritten to need fewer FP64
                                     instructions (lazy scaling, phase pushing); equal to
-                                    the exact mode up to rounding, not bit-identical     */
+                                    the exact mode up to rounding, not bit-identical (a
+                                    gate leaves in each amplitude an error of a few 2^-53
+                                    of the magnitudes that it adds up there)             */
 #define SPZ_EXEC_TMA 32u         /* fused tile passes load each tile with the Tensor
                                     Memory Accelerator (gathers of four 64-byte rows)
                                     instead of thread loads; same results               */

@@ -106,12 +106,6 @@ __device__ __forceinline__ void tile_swap_op(const TileGate& g, Walk W, double* 
 
 // Fast-mode ops in FP64, for the tiles that fixed point cannot hold (the fast
 // mode's own code is tile_fixed.cuh).
-__device__ __forceinline__ void phase_mul(const double2& w, double& r, double& i) {
-  const double x = r, y = i;
-  r = dfma(x, w.x, dmul(dneg(y), w.y));
-  i = dfma(x, w.y, dmul(y, w.x));
-}
-
 // Lazy op, s1 first multiplied by its phase entry when the op has a table.
 static __device__ void tile_lazy_op(const TileGate& g, Walk W, const double2* __restrict__ tab, double* sre,
                                     double* sim, uint32_t n) {
@@ -443,7 +437,7 @@ __device__ __forceinline__ uint32_t fx_pass_gates(const PassArgs& A, uint64_t ba
             const TileGate& h = A.gates[ri];
             if ((base & h.g_ones) != h.g_ones || (base & h.g_zeros) != 0) continue;
             if (h.cond >= 0 && A.outcomes[h.cond] == 0) continue;
-            fx_run_gate<R>(h, A.fxtables, base, e, row);
+            fx_run_gate<R>(h, A.fxtables, A.tables, base, e, row);
           }
 #pragma unroll
           for (int u = 0; u < R; ++u)
@@ -461,7 +455,7 @@ __device__ __forceinline__ uint32_t fx_pass_gates(const PassArgs& A, uint64_t ba
       continue;
     }
     if (g.mode == TM_DIAG_GLOBAL && g.kind != SPZ_GATE_RZ && !(base & g.g_tbit)) continue;
-    fx_tile_gate(g, A.fxtables, base, x, S, T);
+    fx_tile_gate(g, A.fxtables, A.tables, base, x, S, T);
     __syncthreads();
   }
   return x;
@@ -917,7 +911,7 @@ TileGate tile_gate(const GateApp& g, const std::vector<int>& local, const std::v
   if (g.kind >= FK_LAZY_H && g.kind <= FK_LAZY_RY_B) {
     const FxLazy x = fx_lazy(g.kind, g.c.cs);
     t.fx1 = fx_coef(std::isfinite(x.t) ? x.t : 0.0);
-    t.fxswaps = x.swap ? 1u : 0u;
+    t.fxswaps = (x.swap ? 1u : 0u) | (x.t < kFxMinT ? FX_BY_DOUBLE : 0u);
     t.fxturns = x.turns(0) | (x.turns(1) << 2) | ((uint32_t)x.pre << 8);
   }
   if (g.kind == FK_PHASE) {  // elementwise; any qubits (the global index is formed per amplitude)
@@ -1087,11 +1081,13 @@ const PhaseTable& table_of(const GateApp& g, const std::vector<PhaseTable>& tabl
   return g.table >= 0 ? tables[g.table] : unit;
 }
 
-// Whether b can follow a in one TM_LAZY2 op.
+// Whether b can follow a in one TM_LAZY2 op.  The amplitude that both rotations
+// reach is a block's largest times t1 t2 in the worst case: that has to be kFxMinT
+// at least (fixed_point.cuh).
 bool lazy_pair_fits(const GateApp& a, const GateApp& b, const std::vector<PhaseTable>& tables) {
   if (!lazy_uncontrolled(a) || !lazy_uncontrolled(b) || a.target == b.target) return false;
   const PhaseTable &T1 = table_of(a, tables), &T2 = table_of(b, tables);
-  bool ok = T1.m + T2.m <= kPhaseMaxTerms;
+  bool ok = T1.m + T2.m <= kPhaseMaxTerms && fx_lazy(a.kind, a.c.cs).t * fx_lazy(b.kind, b.c.cs).t >= kFxMinT;
   for (int j = 0; ok && j < T2.m; ++j) ok = ((T2.mask[j] >> a.target) & 1) == 0;
   return ok;
 }
@@ -1101,7 +1097,7 @@ bool lazy_pair_fits(const GateApp& a, const GateApp& b, const std::vector<PhaseT
 // the lazy op down to it.  A gate is paired at most once and a paired gate is
 // never moved by itself again, so every step either goes on by a gate or pairs
 // two: the work is at most kReach tests per gate.  (30-qubit brickwork, 20
-// layers: 269 pairs instead of 261; few more fit, a layer's gates inside one
+// layers: 224 pairs, 269 but for kFxMinT; few more fit, a layer's gates inside one
 // pass being an odd number.)
 void order_lazy_pairs(std::vector<GateApp>* gates, const std::vector<PhaseTable>& tables) {
   if (!fast_pairs_enabled()) return;

@@ -4,21 +4,29 @@
 // What bounds the fast mode is DFMA issue (a warp's FP64 instruction holds the
 // SM's FP64 unit for 16 cycles), and its ops may round differently, so they
 // need no IEEE operation each.  For the length of a tile pass an amplitude is
-// (re, im) x 2^(exp - 1080): two 64-bit integers below 2^59 on one exponent.
-// An op brings the amplitudes that it mixes to the largest of their exponents;
+// (re, im) x 2^(exp - 1084): two 64-bit integers on one exponent, the larger of
+// them with its top bit at 61 (fx_settle).  An op brings the amplitudes that it
+// mixes to the largest of their exponents, a few bits lower to leave it room;
 // a multiply-add by a coefficient of magnitude <= 1 is then three 32 x 32-bit
-// multiplies (1.0-1.3 cycles each), with no rounding, packing or normalising
-// between the ops of a pass.
+// multiplies (1.0-1.3 cycles each), with no rounding or packing between the
+// ops of a pass.
 //
-// Precision: an op leaves an error of about 2^-58 of the largest amplitude
-// that it mixes, where FP64 rounds every operation to 2^-53 of its result.  The
-// amplitudes become FP64 again, rounded to nearest, when the pass stores them.
-// Tiles with a component that is not finite or a nonzero amplitude outside
-// [2^-895, 2^600) are worked on in FP64 (fx_in_range).
+// Precision: an op leaves an error of about 2^-58 of the largest amplitude that
+// it mixes, where FP64 rounds every operation to 2^-53 of its result.  So an
+// amplitude that comes out 2^-5 of the largest or more (what a rotation by
+// t >= 2^-5 makes of it, kFxMinT) is as accurate as in FP64; rotations by less go
+// through FP64 one by one, each amplitude back on an exponent of its own
+// (fx_lazy_by_double).  The error is one of the amplitude, shared by its real and
+// imaginary part.  (29-qubit brickwork, 10 layers: 668 ms; 646 without kFxMinT's
+// rules, 617 with one exponent left on the amplitudes of an op, small ones too.)  The amplitudes become FP64 again, rounded to nearest, when the
+// pass stores them.  Tiles with a component that is not finite or a nonzero
+// amplitude outside [2^-895, 2^600) are worked on in FP64 (fx_in_range).
 //
-// Bounds.  An op's inputs have components below 2^59: a phase leaves them below
-// 2^59.5, a rotation below 2^60.5, a second one below 2^61.5; the limbs need
-// inputs below 2^61.  fx_shift then brings them below 2^59 again.
+// Bounds.  The limbs need inputs below 2^61 - 2^29 (the upper one is rounded up),
+// an op's results have to stay below 2^62, and a phase times a component below B
+// gives one below sqrt(2) B, a rotation after it below 2 sqrt(2) B, a second one
+// below 4 sqrt(2) B.  So two rotations start from components below 2^59 (kFxRoom2),
+// one rotation or a phase from below 2^60 (kFxRoom1).
 #pragma once
 
 #include <math.h>
@@ -44,6 +52,9 @@ struct FxAmp {
   int32_t e;
 };
 
+constexpr int kFxRoom2 = 3, kFxRoom1 = 2;  // bits below 2^62 that an op's inputs leave free
+constexpr double kFxMinT = 0x1p-5;
+
 // A coefficient c, |c| <= 1 (and a rounding more), as (h 2^32 + l) / 2^62.
 struct FxCoef {
   int32_t h, l;
@@ -55,7 +66,7 @@ inline FxCoef fx_coef(double c) {
   return FxCoef{(int32_t)((v - l) >> 32), l};
 }
 
-// 4 y = h 2^32 + l, |y| < 2^61
+// 4 y = h 2^32 + l, |y| < 2^61 - 2^29
 struct FxLimb {
   int32_t h, l;
 };
@@ -69,16 +80,16 @@ SPZ_HD int32_t fx_mulhi(int32_t a, int32_t b) { return (int32_t)(((int64_t)a * b
 SPZ_HD int64_t fx_mad(int32_t a, int32_t b, int64_t c) { return (int64_t)a * b + c; }
 
 // x + c y = x + 4 y c 2^62 / 2^64: of the cross products only the upper words are
-// formed, the product of the two low limbs (below the last bit) is left out.
-// (Unsigned low limbs, two instructions to split instead of four, measured 10%
-// slower; 64-bit cross products 2% slower.)
+// formed (each rounded down: the 1 makes up for it), the product of the two low
+// limbs (below the last bit) is left out.  (Unsigned low limbs, two instructions to
+// split instead of four, measured 10% slower; 64-bit cross products 2% slower.)
 SPZ_HD int64_t fx_mac(int64_t x, const FxLimb& y, const FxCoef& c) {
-  return fx_mad(y.h, c.h, x) + (fx_mulhi(y.l, c.h) + fx_mulhi(y.h, c.l));
+  return fx_mad(y.h, c.h, x) + (fx_mulhi(y.l, c.h) + fx_mulhi(y.h, c.l) + 1);
 }
 
 // x - c y
 SPZ_HD int64_t fx_msub(int64_t x, const FxLimb& y, const FxCoef& c) {
-  return fx_mad(y.h, -c.h, x) - (fx_mulhi(y.l, c.h) + fx_mulhi(y.h, c.l));
+  return fx_mad(y.h, -c.h, x) - (fx_mulhi(y.l, c.h) + fx_mulhi(y.h, c.l) + 1);
 }
 
 // (r, i) *= (x, y)
@@ -128,12 +139,14 @@ SPZ_HD void fx_swap(FxAmp& a, FxAmp& b) {
   b = t;
 }
 
-// Bring a[0 .. N-1] to the largest of their exponents, which is returned.
-template <int N>
+// Bring a[0 .. N-1] to the largest of their exponents and ROOM bits down; returns
+// the exponent that they are on then.
+template <int N, int ROOM>
 SPZ_HD int32_t fx_align(FxAmp* a) {
   int32_t E = a[0].e;
 #pragma unroll
   for (int j = 1; j < N; ++j) E = a[j].e > E ? a[j].e : E;
+  E += ROOM;
 #pragma unroll
   for (int j = 0; j < N; ++j) {
     a[j].r = fx_shr(a[j].r, E - a[j].e);
@@ -142,28 +155,31 @@ SPZ_HD int32_t fx_align(FxAmp* a) {
   return E;
 }
 
-// Shift a[0 .. N-1], on exponent E, below 2^59 again.
-template <int N>
-SPZ_HD void fx_settle(FxAmp* a, int32_t E) {
-  uint32_t top = 0;
-#pragma unroll
-  for (int j = 0; j < N; ++j) {
-    const int32_t r = (int32_t)(a[j].r >> 32), i = (int32_t)(a[j].i >> 32);
-    const uint32_t ar = (uint32_t)(r < 0 ? -r : r), ai = (uint32_t)(i < 0 ? -i : i);
-    top = ar > top ? ar : top;
-    top = ai > top ? ai : top;
+SPZ_HD int32_t fx_clz(uint32_t v) {
+#ifdef __CUDA_ARCH__
+  return __clz((int)v);
+#else
+  return v ? __builtin_clz(v) : 32;
+#endif
+}
+
+// a, below 2^62 on exponent E, shifted up so that its larger component has its
+// top bit at 61 (a zero amplitude: on kFxZeroExp).  The upper words say by how
+// much; those of an amplitude below 2^32 (after a cancellation) are shifted in first.
+SPZ_HD void fx_settle(FxAmp& a, int32_t E) {
+  const int32_t r = (int32_t)(a.r >> 32), i = (int32_t)(a.i >> 32);
+  uint32_t m = (uint32_t)((r ^ (r >> 31)) | (i ^ (i >> 31)));
+  if (m == 0u) {
+    a.r <<= 30;
+    a.i <<= 30;
+    E = (a.r | a.i) == 0 ? kFxZeroExp : E - 30;
+    const int32_t r2 = (int32_t)(a.r >> 32), i2 = (int32_t)(a.i >> 32);
+    m = (uint32_t)((r2 ^ (r2 >> 31)) | (i2 ^ (i2 >> 31)) | 1);
   }
-  if (top >= (1u << 27) - 1u) {  // |v| may reach 2^59 .. 2^61.5: 1 to 3 bits
-    const int32_t s = top < (1u << 28) - 1u ? 1 : top < (1u << 29) - 1u ? 2 : 3;
-    E += s;
-#pragma unroll
-    for (int j = 0; j < N; ++j) {
-      a[j].r >>= s;
-      a[j].i >>= s;
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < N; ++j) a[j].e = E;
+  const int32_t d = fx_clz(m) - 2;
+  a.r <<= d;
+  a.i <<= d;
+  a.e = E - d;
 }
 
 // The bits of an amplitude's components as FxAmp (any finite normal numbers; a
@@ -176,7 +192,7 @@ SPZ_HD FxAmp fx_from(uint64_t re, uint64_t im) {
 #pragma unroll
   for (int j = 0; j < 2; ++j) {
     const uint32_t h = (uint32_t)(b[j] >> 32);
-    const uint64_t m = (((uint64_t)((h & 0x000FFFFFu) | 0x00100000u) << 32) | (uint32_t)b[j]) << 5;
+    const uint64_t m = (((uint64_t)((h & 0x000FFFFFu) | 0x00100000u) << 32) | (uint32_t)b[j]) << 9;
     const int32_t f = (int32_t)((h >> 20) & 0x7FFu);
     const int64_t s = (int64_t)((int32_t)h >> 31);
     v[j] = f == 0 ? 0 : ((fx_shr((int64_t)m, e - f) ^ s) - s);
@@ -191,7 +207,7 @@ SPZ_HD bool fx_in_range(uint64_t re, uint64_t im) {
   return big - kFxMinHi < kFxMaxHi - kFxMinHi || ((re | im) << 1) == 0;
 }
 
-// v 2^(E - 1080) as FP64 bits, rounded to nearest, for 64 <= E < 1980.
+// v 2^(E - 1084) as FP64 bits, rounded to nearest, for 64 <= E < 1980.
 SPZ_HD uint64_t fx_bits(int64_t v, int32_t E) {
   const int64_t s = v >> 63;
   const uint64_t a = (uint64_t)((v ^ s) - s);
@@ -206,7 +222,7 @@ SPZ_HD uint64_t fx_bits(int64_t v, int32_t E) {
   const uint64_t n = a ? a << (189u - q) : 0;
 #endif
   const uint64_t m = (n + 0x200u) >> 10;
-  uint32_t hi = (uint32_t)(m >> 32) + ((q + (uint32_t)(E - 185)) << 20);  // E + (q - 127 - 57) - 1
+  uint32_t hi = (uint32_t)(m >> 32) + ((q + (uint32_t)(E - 189)) << 20);  // E + (q - 127 - 61) - 1
   hi |= (uint32_t)s & 0x80000000u;
   hi = a ? hi : 0u;
   return ((uint64_t)hi << 32) | (uint32_t)m;
