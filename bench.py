@@ -85,6 +85,48 @@ def workload_config(n: int, layers: int) -> dict:
             "l2": "inputs larger than L2 (16 GiB state vs 129 MB L2); no flush"}
 
 
+# What the headline line keeps of its longer objects: a line of a few KB is read
+# whole wherever it goes (with a row per gate and target in it, it was 60 KB and
+# was not).  `--detail FILE` writes every object in full.
+HEADLINE = {
+    "roofline": ["bound", "kernel", "achieved", "peak", "unit", "frac", "traffic", "peak_source"],
+    "fp64": ["achieved", "peak", "unit", "frac"],
+    "parity": ["max_abs_diff_fast_vs_exact", "bound", "ok", "exact_ms_per_step", "vs_oracle"],
+    "e2e": ["value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step", "ms_per_step", "upload_alone_ms",
+            "download_alone_ms", "api"],
+    "adjoint": ["qubits", "params", "mode", "adjoint_s", "adjoint_exact_s", "grads_per_s", "speedup_vs_fd",
+                "max_abs_grad_diff_fast_vs_exact"],
+    "batch": ["instances", "seconds_per_batch", "grads_per_s", "speedup_vs_loop", "max_abs_grad_diff_vs_loop"],
+    "qft20": ["program_fast_ms", "program_ms", "execute_ms", "bit_identical"],
+    "measure28": ["sample_ms", "expectation_ms", "shots_bit_identical_vs_oracle", "energy_abs_diff_vs_oracle"],
+    "sweep30": ["summary"],
+    "sweep33": ["summary"],
+}
+
+
+def headline(line: dict) -> dict:
+    """`line` with its longer objects cut down to HEADLINE's keys, their numbers to
+    six digits, and a sweep to each gate's median ms and share of the HBM rate."""
+    def short(v):
+        if isinstance(v, float):
+            return float(f"{v:.6g}")
+        if isinstance(v, dict):
+            return {k: short(w) for k, w in v.items()}
+        return v
+
+    out = dict(line)
+    for key, keep in HEADLINE.items():
+        full = line.get(key)
+        if full is None:
+            continue
+        if key.startswith("sweep"):
+            out[key] = {g: [short(s["ms_median"]), float(f"{s.get('hbm_frac_median', s.get('frac_median')):.3g}")]
+                        for g, s in full["summary"].items()}
+        else:
+            out[key] = {k: full[k] if key == "e2e" else short(full[k]) for k in keep if k in full}
+    return out
+
+
 def replica_throughput(ms_local: float, units_per_replica: float, steps: int, dist=None, device=None):
     """Replicas only: every rank runs the whole workload on its own GPU, no
     data-path collective.  Returns (ms, value): the slowest rank's time (max
@@ -485,8 +527,7 @@ def gpu_arm(args) -> None:
                "upload_alone_ms": 1e3 * (t2 - t1), "download_alone_ms": 1e3 * (t3 - t2),
                "h2d_gbs": 16 * N / (t2 - t1) / 1e9, "d2h_gbs": 16 * N / (t3 - t2) / 1e9,
                "h2d_gbs_torch_copy": 16 * N / min(tup) / 1e9, "host": numa,
-               "api": "spz_circuit_execute_host (pinned host arrays in and out; the copies overlap the leading "
-                      "and trailing tile passes, slab by slab)"}
+               "api": "spz_circuit_execute_host (pinned host arrays in and out)"}
         del hin_re, hin_im, hout_re, hout_im
 
     # Parity at full size: the exact (reference-arithmetic, bit-identical to the
@@ -562,9 +603,8 @@ def gpu_arm(args) -> None:
             "vs_baseline": None, "dtype": "f64", "data": "synthetic",
             "config": workload_config(n, layers),
             "staging": args.staging,
-            "executor": ("fused shared-memory tile passes, exact reference arithmetic" if args.exact else
-                         "fused shared-memory tile passes, fast arithmetic (lazy scaling, U = P RY P, phases pushed "
-                         "through permutations); equal to exact up to rounding"),
+            "executor": "fused tile passes, " + ("exact arithmetic" if args.exact else
+                                                 "fast arithmetic; equal to exact up to rounding"),
             "parallelism": "replicas" if world > 1 else "single-gpu",
             "gates_per_s": len(ops) * world * args.steps / (ms / 1e3),
             "passes_per_step": int(launches / args.steps) - 1,
@@ -593,7 +633,9 @@ def gpu_arm(args) -> None:
             "measure28": mea,
             "sweep33": sw33,
         }
-        print(json.dumps(line), flush=True)
+        if args.detail:
+            Path(args.detail).write_text(json.dumps(line))
+        print(json.dumps(headline(line)), flush=True)
     if dist:
         dist.destroy_process_group()
 
@@ -989,6 +1031,8 @@ def main() -> None:
     ap.add_argument("--no-parity", action="store_true")
     ap.add_argument("--no-sweep", action="store_true", help="skip the per-gate sweep at the headline's qubit count")
     ap.add_argument("--no-sweep33", action="store_true", help="skip the per-gate sweep at 33 qubits (128 GiB)")
+    ap.add_argument("--detail", default="", metavar="FILE",
+                    help="write every object of the headline line in full to FILE (per-target sweep rows among them)")
     ap.add_argument("--exact", action="store_true", help="time the bit-exact executor mode instead of fast mode")
     ap.add_argument("--staging", default="threads", choices=["threads", "tma", "tma-prefetch", "shuffle"],
                     help="how fused passes stage their tiles: thread loads (default), TMA gathers, or "
