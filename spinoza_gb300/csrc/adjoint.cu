@@ -468,21 +468,13 @@ int apply_hamiltonian(spz_state_t h, const spz_pauli_term* terms, size_t nterms,
   }
   if (diag.size() > (size_t)kHpMaxDiag) return fail(SPZ_ERR_UNSUPPORTED, "more than 64 diagonal terms");
   const size_t nch = (diag.size() + 7) / 8;
-  // Entry v of a chunk: sum of its coefficients, negated where v has the bit.  (Not
-  // a constant plus corrections: the constant's rounding would shift every
-  // amplitude's value alike, and with it the energy.)
   std::vector<double> tab(std::max<size_t>(1, nch * 256), 0.0);
-  for (size_t ch = 0; ch < nch; ++ch)
-    for (int v = 0; v < 256; ++v) {
-      double hi = 0.0, lo = 0.0;
-      for (int b = 0; b < 8 && ch * 8 + b < diag.size(); ++b) {
-        const double c = ((v >> b) & 1) ? -terms[diag[ch * 8 + b]].coeff : terms[diag[ch * 8 + b]].coeff;
-        const double t = hi + c, z = t - hi;  // two-sum
-        lo += (hi - (t - z)) + (c - z);
-        hi = t;
-      }
-      tab[ch * 256 + v] = hi + lo;
-    }
+  for (size_t ch = 0; ch < nch; ++ch) {
+    double c8[8];
+    const int count = (int)std::min<size_t>(8, diag.size() - ch * 8);
+    for (int b = 0; b < count; ++b) c8[b] = terms[diag[ch * 8 + b]].coeff;
+    for (int v = 0; v < 256; ++v) tab[ch * 256 + v] = signed_sum(c8, count, v);
+  }
   void* scratch;
   int rc = ensure_dev_scratch(h, tab.size() * sizeof(double), &scratch);
   if (rc) return rc;

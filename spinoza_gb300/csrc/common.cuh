@@ -249,6 +249,21 @@ struct GateApp {
 void lower_fast(const std::vector<GateApp>& in, uint32_t n, std::vector<GateApp>* out,
                 std::vector<PhaseTable>* tables);
 
+// c[0] .. c[count - 1] added up, each negated where v has its bit, the roundings of
+// the partial sums carried along (two-sums).  Entries of diagonal terms' tables:
+// not a constant plus corrections, whose rounding would shift every amplitude's
+// value alike, and with it an energy.
+inline double signed_sum(const double* c, int count, int v) {
+  double hi = 0.0, lo = 0.0;
+  for (int b = 0; b < count; ++b) {
+    const double x = ((v >> b) & 1) ? -c[b] : c[b];
+    const double t = hi + x, z = t - hi;
+    lo += (hi - (t - z)) + (x - z);
+    hi = t;
+  }
+  return hi + lo;
+}
+
 // Validate and build a GateApp (returns a status).
 int make_gate_app(uint32_t n, const spz_gate& g, uint32_t target, uint64_t ones, uint64_t zeros,
                   GateApp* out);

@@ -414,9 +414,9 @@ __global__ void __launch_bounds__(kRedThreads) x_pauli_kernel(const double* __re
 // One pass loads a tile of 2^k amplitudes (all values of k local qubits) into
 // shared memory and accumulates, per thread:
 //  * (first pass only) the diagonal terms: with w_k = parity(x & z_k), the
-//    diagonal part is D(x) = C + sum_j T_j[w bits 8j..8j+7], T_j 256-entry tables
-//    of -2 sum c_k over the set bits, so a whole Ising-type chain costs a few
-//    FP64 operations per amplitude; energy += |psi_x|^2 D(x);
+//    diagonal part is D(x) = sum_j T_j[w bits 8j..8j+7], T_j 256-entry tables of
+//    the eight terms' signed sums, so a whole Ising-type chain costs a few FP64
+//    operations per amplitude; energy += |psi_x|^2 D(x);
 //  * every X/Y-type term whose X-mask lies in the tile: per pair (x, x ^ xmask)
 //    the pair's contribution to Re<psi|P|psi>, one accumulator per term.
 // Each term's accumulators are reduced once at the end (fixed order).
@@ -450,7 +450,6 @@ struct PtArgs {
   // The chunk index w(x) = sum_j parity(x & dz_j) << j is linear over GF(2):
   // w(base | e) = w(base) ^ L0[e & 63] ^ L1[e >> 6] for the tile offset e.
   uint8_t lz[kPtMaxDiag / 8][2][64];
-  double dconst;             // C = sum of the diagonal coefficients
   int nt;
   PtTerm t[kPtMaxTerms];
   double* partials;          // (nt + 1) x gridDim.x
@@ -499,13 +498,13 @@ __global__ void __launch_bounds__(kPtThreads) pauli_tile_kernel(PtArgs A) {
         }
       }
       for (uint32_t e = threadIdx.x; e < T; e += blockDim.x) {
-        double d = A.dconst;
+        double d = 0.0;
         const uint32_t e0 = e & 63, e1 = (e >> 6) & 63;
 #pragma unroll
         for (int ch = 0; ch < kPtMaxDiag / 8; ++ch) {
           if (ch >= nch) break;
-          const uint32_t w = wb[ch] ^ slz[ch * 128 + e0] ^ slz[ch * 128 + 64 + e1];
-          d = dadd(d, stab[ch * 256 + w]);
+          const double v = stab[ch * 256 + (wb[ch] ^ slz[ch * 128 + e0] ^ slz[ch * 128 + 64 + e1])];
+          d = ch == 0 ? v : dadd(d, v);
         }
         const double a = sre[e], b = sim[e];
         acc[kPtMaxTerms] = dfma(dfma(a, a, dmul(b, b)), d, acc[kPtMaxTerms]);
@@ -612,15 +611,12 @@ static int pauli_tiles(spz_state_t h, const spz_pauli_term* terms, size_t nterms
   const size_t nd = diag.size();
   const size_t nchunks = (nd + 7) / 8;
   std::vector<double> tab(std::max<size_t>(1, nchunks) * 256, 0.0);
-  double dconst = 0.0;
-  for (size_t j = 0; j < nd; ++j) dconst += terms[diag[j]].coeff;
-  for (size_t ch = 0; ch < nchunks; ++ch)
-    for (int v = 0; v < 256; ++v) {
-      double s = 0.0;
-      for (int b = 0; b < 8 && ch * 8 + b < nd; ++b)
-        if ((v >> b) & 1) s += -2.0 * terms[diag[ch * 8 + b]].coeff;
-      tab[ch * 256 + v] = s;
-    }
+  for (size_t ch = 0; ch < nchunks; ++ch) {
+    double c[8];
+    const int count = (int)std::min<size_t>(8, nd - ch * 8);
+    for (int b = 0; b < count; ++b) c[b] = terms[diag[ch * 8 + b]].coeff;
+    for (int v = 0; v < 256; ++v) tab[ch * 256 + v] = signed_sum(c, count, v);
+  }
   const int blocks = (int)std::min<uint64_t>(1ull << (n - k), (uint64_t)kNumSMs * 3);
   const size_t slots_per_pass = (size_t)(kPtMaxTerms + 1) * blocks;
   const size_t nres = passes.size() * (kPtMaxTerms + 1);
@@ -659,7 +655,6 @@ static int pauli_tiles(spz_state_t h, const spz_pauli_term* terms, size_t nterms
       A.ndiag = (int)nd;
       for (size_t j = 0; j < nd; ++j) A.dz[j] = terms[diag[j]].z_mask;
       A.dtab = dtab;
-      A.dconst = dconst;
       // column of tile-offset bit b in chunk ch: the chunk's terms whose Z-mask
       // holds the local qubit lpos[b]
       for (int ch = 0; ch < (int)((nd + 7) / 8); ++ch) {
