@@ -174,10 +174,11 @@ struct PairGate {
 
 // Diagonal gates on one amplitude; `one` is the amplitude's target bit.  RZ's
 // entries are (re, im) = (cos, -sin) on 0 and (cos, sin) on 1.
-// ZEROS: amplitudes that are zero stay on the integer path (the per-gate kernels,
-// which HBM bounds; 25 qubits, real-valued state: RZ 366 us without, 178 with, P
-// 147 and 98).  In tile passes, where the integer pipes are the busier ones, the
-// tests cost more than they give (20-qubit QFT 632 us without, 674 with).
+// ZEROS: warps with amplitudes that are zero have an integer path too (the
+// per-gate kernels, which HBM bounds; 25 qubits, real-valued state: RZ 366 us
+// without, 178 with, P 147 and 98).  In tile passes, where the integer pipes are
+// the busier ones, it costs more than it gives (20-qubit QFT 632 us without, 674
+// with it for every warp).
 template <int KIND, bool ZEROS = false>
 struct DiagGate : DiagCoef {
   __device__ __forceinline__ explicit DiagGate(const DiagCoef& d) : DiagCoef(d) {}
@@ -188,15 +189,21 @@ struct DiagGate : DiagCoef {
     }
   }
 
-  // Whether the amplitude's products may come from the integer pipes.
+  // The products' ways: FP64, integer, integer with zeros.
+  enum Way { FP = 0, INT = 1, INT_ZERO = 2 };
+
+  // Whether the amplitude's products may take the way W.
+  template <Way W>
   __device__ __forceinline__ bool fits(double re, double im) const {
-    const auto ok = [this](double y) { return ZEROS ? mul_ok_or_zero(dbits(y), range) : mul_ok(dbits(y), range); };
+    const auto ok = [this](double y) {
+      return W == INT_ZERO ? mul_ok_or_zero(dbits(y), range) : mul_ok(dbits(y), range);
+    };
     if constexpr (KIND == SPZ_GATE_P) return ok(re) & ok(im);
     else if constexpr (KIND == SPZ_GATE_RZ) return ok(im);
     else return true;
   }
 
-  template <bool INT>
+  template <Way W>
   __device__ __forceinline__ void apply(bool one, double& re, double& im) const {
     if constexpr (KIND == SPZ_GATE_Z) {  // z_proc_chunk, gates.rs:1054-1056
       if (one) { re = dneg(re); im = dneg(im); }
@@ -204,8 +211,8 @@ struct DiagGate : DiagCoef {
       if (one) {
         const double zr = re, zi = im;
         double is, rs;  // -im * sin, re * sin
-        if constexpr (!INT) { is = dmul(dneg(zi), im1); rs = dmul(zr, im1); }
-        else if constexpr (ZEROS) { is = imul_or_zero(zi, mul_flip(mim, true)); rs = imul_or_zero(zr, mim); }
+        if constexpr (W == FP) { is = dmul(dneg(zi), im1); rs = dmul(zr, im1); }
+        else if constexpr (W == INT_ZERO) { is = imul_or_zero(zi, mul_flip(mim, true)); rs = imul_or_zero(zr, mim); }
         else { is = dneg(imul(zi, mim)); rs = imul(zr, mim); }
         re = dfma(zr, re1, is);
         im = dfma(zi, re1, rs);
@@ -213,8 +220,8 @@ struct DiagGate : DiagCoef {
     } else if constexpr (KIND == SPZ_GATE_RZ) {  // rz_apply_strategy1, gates.rs:939-946
       const double cr = re, ci = im, s = flip_sign(im1, !one);
       double is, ic;  // -im * the entry's sin, im * cos
-      if constexpr (!INT) { is = dmul(dneg(ci), s); ic = dmul(ci, re1); }
-      else if constexpr (ZEROS) { is = imul_or_zero(ci, mul_flip(mim, one)); ic = imul_or_zero(ci, mre); }
+      if constexpr (W == FP) { is = dmul(dneg(ci), s); ic = dmul(ci, re1); }
+      else if constexpr (W == INT_ZERO) { is = imul_or_zero(ci, mul_flip(mim, one)); ic = imul_or_zero(ci, mre); }
       else { is = flip_sign(imul(ci, mim), one); ic = imul(ci, mre); }
       re = dfma(cr, re1, is);
       im = dfma(cr, s, ic);
@@ -222,18 +229,22 @@ struct DiagGate : DiagCoef {
   }
 
   __device__ __forceinline__ void operator()(bool one, double& re, double& im) const {
-    if (warp_all(fits(re, im))) apply<true>(one, re, im);
-    else apply<false>(one, re, im);
+    if (warp_all(fits<INT>(re, im))) apply<INT>(one, re, im);
+    else if (ZEROS && warp_all(fits<INT_ZERO>(re, im))) apply<INT_ZERO>(one, re, im);
+    else apply<FP>(one, re, im);
   }
 
   // Two amplitudes of a thread, their instructions side by side.
   __device__ __forceinline__ void operator()(bool one0, double& re0, double& im0, bool one1, double& re1, double& im1) const {
-    if (warp_all(fits(re0, im0) & fits(re1, im1))) {
-      apply<true>(one0, re0, im0);
-      apply<true>(one1, re1, im1);
+    if (warp_all(fits<INT>(re0, im0) & fits<INT>(re1, im1))) {
+      apply<INT>(one0, re0, im0);
+      apply<INT>(one1, re1, im1);
+    } else if (ZEROS && warp_all(fits<INT_ZERO>(re0, im0) & fits<INT_ZERO>(re1, im1))) {
+      apply<INT_ZERO>(one0, re0, im0);
+      apply<INT_ZERO>(one1, re1, im1);
     } else {
-      apply<false>(one0, re0, im0);
-      apply<false>(one1, re1, im1);
+      apply<FP>(one0, re0, im0);
+      apply<FP>(one1, re1, im1);
     }
   }
 };
