@@ -106,6 +106,12 @@ __device__ __forceinline__ void tile_swap_op(const TileGate& g, Walk W, double* 
 
 // Fast-mode ops in FP64, for the tiles that fixed point cannot hold (the fast
 // mode's own code is tile_fixed.cuh).
+__device__ __forceinline__ void phase_mul(const double2& w, double& r, double& i) {
+  const double x = r, y = i;
+  r = dfma(x, w.x, dmul(dneg(y), w.y));
+  i = dfma(x, w.y, dmul(y, w.x));
+}
+
 // Lazy op, s1 first multiplied by its phase entry when the op has a table.
 static __device__ void tile_lazy_op(const TileGate& g, Walk W, const double2* __restrict__ tab, double* sre,
                                     double* sim, uint32_t n) {
@@ -437,7 +443,7 @@ __device__ __forceinline__ uint32_t fx_pass_gates(const PassArgs& A, uint64_t ba
             const TileGate& h = A.gates[ri];
             if ((base & h.g_ones) != h.g_ones || (base & h.g_zeros) != 0) continue;
             if (h.cond >= 0 && A.outcomes[h.cond] == 0) continue;
-            fx_run_gate<R>(h, A.fxtables, A.tables, base, e, row);
+            fx_run_gate<R>(h, A.fxtables, base, e, row);
           }
 #pragma unroll
           for (int u = 0; u < R; ++u)
@@ -455,7 +461,7 @@ __device__ __forceinline__ uint32_t fx_pass_gates(const PassArgs& A, uint64_t ba
       continue;
     }
     if (g.mode == TM_DIAG_GLOBAL && g.kind != SPZ_GATE_RZ && !(base & g.g_tbit)) continue;
-    fx_tile_gate(g, A.fxtables, A.tables, base, x, S, T);
+    fx_tile_gate(g, A.fxtables, base, x, S, T);
     __syncthreads();
   }
   return x;
@@ -911,7 +917,12 @@ TileGate tile_gate(const GateApp& g, const std::vector<int>& local, const std::v
   if (g.kind >= FK_LAZY_H && g.kind <= FK_LAZY_RY_B) {
     const FxLazy x = fx_lazy(g.kind, g.c.cs);
     t.fx1 = fx_coef(std::isfinite(x.t) ? x.t : 0.0);
-    t.fxswaps = (x.swap ? 1u : 0u) | (x.t < kFxMinT ? FX_BY_DOUBLE : 0u);
+    t.fxswaps = x.swap ? 1u : 0u;
+    if (x.t < kFxMinT) {  // as t 2^-k, 1/2 <= t < 1 (nothing: k is past every exponent)
+      const int k = x.t > 0.0 ? -std::ilogb(x.t) - 1 : 4096;
+      t.fx1 = fx_coef(std::ldexp(x.t, k));
+      t.fxswaps |= FX_SMALL | (uint32_t)k << kFxSmallShift;
+    }
     t.fxturns = x.turns(0) | (x.turns(1) << 2) | ((uint32_t)x.pre << 8);
   }
   if (g.kind == FK_PHASE) {  // elementwise; any qubits (the global index is formed per amplitude)

@@ -49,7 +49,8 @@ enum TileMode {
 };
 enum MoveKind { MV_X = 0, MV_CX1 = 1, MV_CX0 = 2, MV_SWAP = 3 };
 
-constexpr uint32_t FX_BY_DOUBLE = 0x100u;
+constexpr uint32_t FX_SMALL = 0x100u;
+constexpr int kFxSmallShift = 16;
 
 struct TileGate {
   int32_t kind;
@@ -85,8 +86,8 @@ struct TileGate {
   int32_t run_end;
   // Fast mode in fixed point (tile_fixed.cuh).  A lazy op: its rotation's t
   // (a TM_LAZY2's in fx1 and fx2), bit 0 / 1 of fxswaps: the two members are
-  // swapped before the first / second rotation (FX_BY_DOUBLE: the op goes through
-  // FP64), fxturns bits 2 j, 2 j + 1: the
+  // swapped before the first / second rotation (FX_SMALL: t is fx1 times 2 to
+  // the minus fxswaps >> kFxSmallShift), fxturns bits 2 j, 2 j + 1: the
   // power of i that output j is multiplied by, bits 8, 9: the power of i on s1
   // before the op (of a lazy op without a phase table; a table holds it in its
   // entries).  A phase op: fexp, the power of two of its table.

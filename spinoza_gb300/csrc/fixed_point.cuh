@@ -14,13 +14,14 @@
 // Precision: an op leaves an error of about 2^-58 of the largest amplitude that
 // it mixes, where FP64 rounds every operation to 2^-53 of its result.  So an
 // amplitude that comes out 2^-5 of the largest or more (what a rotation by
-// t >= 2^-5 makes of it, kFxMinT) is as accurate as in FP64; rotations by less go
-// through FP64 one by one, each amplitude back on an exponent of its own
-// (fx_lazy_by_double).  The error is one of the amplitude, shared by its real and
-// imaginary part.  (29-qubit brickwork, 10 layers: 668 ms; 646 without kFxMinT's
-// rules, 617 with one exponent left on the amplitudes of an op, small ones too.)  The amplitudes become FP64 again, rounded to nearest, when the
-// pass stores them.  Tiles with a component that is not finite or a nonzero
-// amplitude outside [2^-895, 2^600) are worked on in FP64 (fx_in_range).
+// t >= 2^-5 makes of it, kFxMinT) is as accurate as in FP64; rotations by less
+// have an exponent for each result (fx_lazy_small).  The error is one of the
+// amplitude, shared by its real and imaginary part; a component that is zero
+// stays zero where the op adds nothing to it.  The amplitudes become FP64 again,
+// rounded to nearest, when the pass stores them.  Tiles with a component that is
+// not finite or a nonzero amplitude outside [2^-895, 2^600) are worked on in FP64
+// (fx_in_range).  (29-qubit brickwork, 10 layers: 662 ms; 637 without kFxMinT's
+// rules, 617 with the amplitudes of an op left on one exponent.)
 //
 // Bounds.  The limbs need inputs below 2^61 - 2^29 (the upper one is rounded up),
 // an op's results have to stay below 2^62, and a phase times a component below B
@@ -80,16 +81,16 @@ SPZ_HD int32_t fx_mulhi(int32_t a, int32_t b) { return (int32_t)(((int64_t)a * b
 SPZ_HD int64_t fx_mad(int32_t a, int32_t b, int64_t c) { return (int64_t)a * b + c; }
 
 // x + c y = x + 4 y c 2^62 / 2^64: of the cross products only the upper words are
-// formed (each rounded down: the 1 makes up for it), the product of the two low
-// limbs (below the last bit) is left out.  (Unsigned low limbs, two instructions to
-// split instead of four, measured 10% slower; 64-bit cross products 2% slower.)
+// formed, the product of the two low limbs (below the last bit) is left out; a zero
+// stays one.  (Unsigned low limbs, two instructions to split instead of four,
+// measured 10% slower; 64-bit cross products 2% slower.)
 SPZ_HD int64_t fx_mac(int64_t x, const FxLimb& y, const FxCoef& c) {
-  return fx_mad(y.h, c.h, x) + (fx_mulhi(y.l, c.h) + fx_mulhi(y.h, c.l) + 1);
+  return fx_mad(y.h, c.h, x) + (fx_mulhi(y.l, c.h) + fx_mulhi(y.h, c.l));
 }
 
 // x - c y
 SPZ_HD int64_t fx_msub(int64_t x, const FxLimb& y, const FxCoef& c) {
-  return fx_mad(y.h, -c.h, x) - (fx_mulhi(y.l, c.h) + fx_mulhi(y.h, c.l) + 1);
+  return fx_mad(y.h, -c.h, x) - (fx_mulhi(y.l, c.h) + fx_mulhi(y.h, c.l));
 }
 
 // (r, i) *= (x, y)
@@ -151,6 +152,7 @@ SPZ_HD int32_t fx_align(FxAmp* a) {
   for (int j = 0; j < N; ++j) {
     a[j].r = fx_shr(a[j].r, E - a[j].e);
     a[j].i = fx_shr(a[j].i, E - a[j].e);
+    if constexpr (N == 1) a[j].e = E;
   }
   return E;
 }
@@ -163,23 +165,38 @@ SPZ_HD int32_t fx_clz(uint32_t v) {
 #endif
 }
 
-// a, below 2^62 on exponent E, shifted up so that its larger component has its
-// top bit at 61 (a zero amplitude: on kFxZeroExp).  The upper words say by how
-// much; those of an amplitude below 2^32 (after a cancellation) are shifted in first.
-SPZ_HD void fx_settle(FxAmp& a, int32_t E) {
+// The larger of an amplitude's upper words without their signs, and the shift that
+// brings its top bit to 29 (the component's to 61; one bit less at some negative
+// powers of two).
+SPZ_HD uint32_t fx_top(const FxAmp& a) {
   const int32_t r = (int32_t)(a.r >> 32), i = (int32_t)(a.i >> 32);
-  uint32_t m = (uint32_t)((r ^ (r >> 31)) | (i ^ (i >> 31)));
-  if (m == 0u) {
-    a.r <<= 30;
-    a.i <<= 30;
-    E = (a.r | a.i) == 0 ? kFxZeroExp : E - 30;
-    const int32_t r2 = (int32_t)(a.r >> 32), i2 = (int32_t)(a.i >> 32);
-    m = (uint32_t)((r2 ^ (r2 >> 31)) | (i2 ^ (i2 >> 31)) | 1);
-  }
-  const int32_t d = fx_clz(m) - 2;
+  return (uint32_t)(r < 0 ? -r : r) | (uint32_t)(i < 0 ? -i : i);
+}
+SPZ_HD void fx_shift_up(FxAmp& a, int32_t E, uint32_t top) {
+  const int32_t d = fx_clz(top) - 2;
   a.r <<= d;
   a.i <<= d;
   a.e = E - d;
+}
+
+// a[0 .. N-1], below 2^62 on exponent E, shifted up so that the larger component of
+// each has its top bit at 61 (a zero amplitude: on kFxZeroExp).  The upper words say
+// by how much; where they are zero (zeros, cancellations) the lower ones are
+// shifted in first.
+template <int N>
+SPZ_HD void fx_settle(FxAmp* a, int32_t E) {
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    uint32_t top = fx_top(a[j]);
+    int32_t e = E;
+    if (top == 0u) {
+      a[j].r <<= 29;
+      a[j].i <<= 29;
+      e = (a[j].r | a[j].i) == 0 ? kFxZeroExp : E - 29;
+      top = fx_top(a[j]) | 1u;
+    }
+    fx_shift_up(a[j], e, top);
+  }
 }
 
 // The bits of an amplitude's components as FxAmp (any finite normal numbers; a

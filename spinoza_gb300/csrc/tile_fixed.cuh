@@ -54,13 +54,6 @@ __device__ __forceinline__ uint32_t fx_index(const TileGate& g, uint32_t bidx, u
   return idx;
 }
 
-// A phase entry times an amplitude in FP64.
-__device__ __forceinline__ void phase_mul(const double2& w, double& r, double& i) {
-  const double x = r, y = i;
-  r = dfma(x, w.x, dmul(dneg(y), w.y));
-  i = dfma(x, w.y, dmul(y, w.x));
-}
-
 // One lazy op on a pair; w: its phase entry (with has_w), fx* from the descriptor.
 __device__ __forceinline__ void fx_lazy_pair(FxAmp* a, const FxCoef& t, bool has_w, const int4& w, uint32_t swaps,
                                              uint32_t turns) {
@@ -73,44 +66,41 @@ __device__ __forceinline__ void fx_lazy_pair(FxAmp* a, const FxCoef& t, bool has
     fx_quarter(a[0], turns);
     fx_quarter(a[1], turns >> 2);
   }
-  fx_settle(a[0], E);
-  fx_settle(a[1], E);
+  fx_settle<2>(a, E);
 }
 
-// The same through FP64, for a rotation by less than kFxMinT (FX_BY_DOUBLE): what it
-// adds to an amplitude may lie so far below the other one that a common exponent
-// would lose it.  w: the op's FP64 phase entry.
-__device__ __forceinline__ void fx_lazy_by_double(const TileGate& g, FxAmp* a, bool has_w, const double2& w) {
-  double2 x = fx_to_double(a[0]), y = fx_to_double(a[1]);
-  if (has_w) phase_mul(w, y.x, y.y);
-  fast_pair_kind(g.kind, g.c.cs, x.x, x.y, y.x, y.y);
-  a[0] = fx_from_double(x.x, x.y);
-  a[1] = fx_from_double(y.x, y.y);
+// The same for a rotation by t 2^-k below kFxMinT, 1/2 <= t < 1 or t = 0 (k above
+// FX_SMALL's shift in `swaps`): what it adds to an amplitude may lie far below the
+// other one, so each result has a common exponent of its own for its two terms.
+__device__ __forceinline__ void fx_lazy_small(FxAmp* a, const FxCoef& t, bool has_w, const int4& w, uint32_t swaps,
+                                              uint32_t turns) {
+  const int32_t k = (int32_t)(swaps >> kFxSmallShift);
+  fx_align<1, kFxRoom1>(a);
+  fx_align<1, kFxRoom1>(a + 1);
+  if (has_w) fx_cmul(a[1].r, a[1].i, FxCoef{w.x, w.y}, FxCoef{w.z, w.w});
+  else fx_quarter(a[1], turns >> 8);
+  if (swaps & 1u) fx_swap(a[0], a[1]);
+  const int32_t e0 = a[0].e, e1 = a[1].e, E0 = max(e0, e1 - k), E1 = max(e1, e0 - k);
+  const FxLimb c = fx_split(fx_shr(a[1].r, E0 + k - e1)), d = fx_split(fx_shr(a[1].i, E0 + k - e1));
+  const FxLimb p = fx_split(fx_shr(a[0].r, E1 + k - e0)), q = fx_split(fx_shr(a[0].i, E1 + k - e0));
+  a[0].r = fx_msub(fx_shr(a[0].r, E0 - e0), c, t);
+  a[0].i = fx_msub(fx_shr(a[0].i, E0 - e0), d, t);
+  a[1].r = fx_mac(fx_shr(a[1].r, E1 - e1), p, t);
+  a[1].i = fx_mac(fx_shr(a[1].i, E1 - e1), q, t);
+  fx_quarter(a[0], turns);
+  fx_quarter(a[1], turns >> 2);
+  fx_settle<1>(a, E0);
+  fx_settle<1>(a + 1, E1);
 }
 
 // A phase entry times one amplitude (2^fexp: the table's scale).
 __device__ __forceinline__ void fx_phase(FxAmp& a, const int4& w, int32_t fexp) {
   const int32_t E = fx_align<1, kFxRoom1>(&a);
   fx_cmul(a.r, a.i, FxCoef{w.x, w.y}, FxCoef{w.z, w.w});
-  fx_settle(a, E + fexp);
+  fx_settle<1>(&a, E + fexp);
 }
 
-static __device__ void fx_tile_lazy_by_double(const TileGate& g, const double2* __restrict__ tables, Walk W,
-                                              const FxTile& S, uint32_t npairs) {
-  const uint32_t tmask = g.tmask;
-  const bool has_w = g.pm > 0;
-  const double2* tab = tables + g.ptab;
-  for (uint32_t m = threadIdx.x, it = 0; m < npairs; m += blockDim.x, ++it) {
-    const uint32_t word = W.word(it), s0 = word & 0xFFFFu, s1 = s0 ^ tmask;
-    FxAmp a[2] = {S.load(s0), S.load(s1)};
-    double2 w = make_double2(1.0, 0.0);
-    if (has_w) w = __ldg(tab + (word >> 16));
-    fx_lazy_by_double(g, a, has_w, w);
-    S.store(s0, a[0]);
-    S.store(s1, a[1]);
-  }
-}
-
+template <bool SMALL>
 static __device__ void fx_tile_lazy(const TileGate& g, const int4* __restrict__ tables, Walk W,
                                     const FxTile& S, uint32_t npairs) {
   const uint32_t tmask = g.tmask, swaps = g.fxswaps, turns = g.fxturns;
@@ -122,7 +112,8 @@ static __device__ void fx_tile_lazy(const TileGate& g, const int4* __restrict__ 
     FxAmp a[2] = {S.load(s0), S.load(s1)};
     int4 w = make_int4(0, 0, 0, 0);
     if (has_w) w = __ldg(tab + (word >> 16));
-    fx_lazy_pair(a, t, has_w, w, swaps, turns);
+    if constexpr (SMALL) fx_lazy_small(a, t, has_w, w, swaps, turns);
+    else fx_lazy_pair(a, t, has_w, w, swaps, turns);
     S.store(s0, a[0]);
     S.store(s1, a[1]);
   }
@@ -161,8 +152,7 @@ static __device__ void fx_tile_lazy2(const TileGate& g, const int4* __restrict__
 #pragma unroll
       for (int j = 0; j < 4; ++j) fx_quarter(a[j], turns >> (2 * j));
     }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) fx_settle(a[j], X);
+    fx_settle<4>(a, X);
     S.store(e, a[0]);
     S.store(e ^ b1, a[1]);
     S.store(e ^ b2, a[2]);
@@ -239,16 +229,15 @@ static __device__ void fx_tile_exact(const TileGate& g, uint64_t base, Walk W, c
   }
 }
 
-// Op g on the tile; x: the tile's (tile_map.cuh), tables64: the phase tables in FP64.
-static __device__ __forceinline__ void fx_tile_gate(const TileGate& g, const int4* __restrict__ tables,
-                                                    const double2* __restrict__ tables64, uint64_t base, uint32_t x,
-                                                    const FxTile& S, uint32_t T) {
+// Op g on the tile; x: the tile's (tile_map.cuh).
+static __device__ __forceinline__ void fx_tile_gate(const TileGate& g, const int4* __restrict__ tables, uint64_t base,
+                                                    uint32_t x, const FxTile& S, uint32_t T) {
   const uint32_t nw = T >> g.npos;
   Walk W(g, x, fx_base_index(g, base));
   if (g.mode == TM_LAZY2) fx_tile_lazy2(g, tables, W, S, nw);
   else if (g.mode == TM_PHASE) fx_tile_phase(g, tables, W, S, nw);
-  else if (g.mode == TM_PAIR && (g.fxswaps & FX_BY_DOUBLE)) fx_tile_lazy_by_double(g, tables64, W, S, nw);
-  else if (g.mode == TM_PAIR && g.kind >= FK_LAZY_H) fx_tile_lazy(g, tables, W, S, nw);
+  else if (g.mode == TM_PAIR && (g.fxswaps & FX_SMALL)) fx_tile_lazy<true>(g, tables, W, S, nw);
+  else if (g.mode == TM_PAIR && g.kind >= FK_LAZY_H) fx_tile_lazy<false>(g, tables, W, S, nw);
   else fx_tile_exact(g, base, W, S, nw);
 }
 
@@ -258,9 +247,8 @@ static __device__ __forceinline__ void fx_tile_gate(const TileGate& g, const int
 // part of a phase index is formed once for the R rows (row by row, a fast QFT of
 // 24 qubits took 8.9 ms; in FP64 7.3).
 template <int R>
-__device__ __forceinline__ void fx_run_gate(const TileGate& g, const int4* __restrict__ tables,
-                                            const double2* __restrict__ tables64, uint64_t base, const uint32_t* e,
-                                            FxAmp* x) {
+__device__ __forceinline__ void fx_run_gate(const TileGate& g, const int4* __restrict__ tables, uint64_t base,
+                                            const uint32_t* e, FxAmp* x) {
   uint32_t idx[R];
   const uint32_t tb = g.mode == TM_PAIR ? g.tbit : 0u;
   if (g.pm > 0) {
@@ -286,14 +274,11 @@ __device__ __forceinline__ void fx_run_gate(const TileGate& g, const int4* __res
       p.i = (int64_t)__shfl_xor_sync(0xffffffffu, (long long)x[u].i, tb);
       p.e = __shfl_xor_sync(0xffffffffu, x[u].e, tb);
       FxAmp a[2] = {hi ? p : x[u], hi ? x[u] : p};
-      if (g.fxswaps & FX_BY_DOUBLE) {
-        double2 w = make_double2(1.0, 0.0);
-        if (g.pm > 0) w = __ldg(tables64 + g.ptab + idx[u]);
-        fx_lazy_by_double(g, a, g.pm > 0, w);
-      } else if (g.kind >= FK_LAZY_H) {
+      if (g.kind >= FK_LAZY_H) {
         int4 w = make_int4(0, 0, 0, 0);
         if (g.pm > 0) w = __ldg(tab + idx[u]);
-        fx_lazy_pair(a, g.fx1, g.pm > 0, w, g.fxswaps, g.fxturns);
+        if (g.fxswaps & FX_SMALL) fx_lazy_small(a, g.fx1, g.pm > 0, w, g.fxswaps, g.fxturns);
+        else fx_lazy_pair(a, g.fx1, g.pm > 0, w, g.fxswaps, g.fxturns);
       } else if ((e[u] & ~tb & g.e_mask) == g.l_ones) {
         fx_exact_pair(g, a[0], a[1]);
       }
