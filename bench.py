@@ -474,7 +474,7 @@ def gpu_arm(args) -> None:
     N = 1 << n
     tile_avg_ms = tile_ms / max(1, tile_launches)
     achieved = (32 * N) / (tile_avg_ms / 1e3) / 1e9
-    traffic = profile_traffic("tile_kernel_brickwork30.txt")
+    traffic = profile_traffic("tile_kernel_fixed_and_exact26.txt")
     fma_rate_after = core.fp64_fma_rate()
     fma_rate = max(fma_rate_before, fma_rate_after)
     fp64_achieved = fp64_ops / ((tile_ms + plain_ms) / 1e3)
