@@ -212,7 +212,7 @@ __global__ void inner_re_kernel(const double* __restrict__ pr, const double* __r
 // 128 threads x 6 blocks per SM (what the tiles' shared memory allows): with the
 // products on the integer pipes 12 warps per SM (64 threads) no longer fill the
 // FP64 pipe.  21 qubits, 6 layers, the six passes: 15.2 ms with DFMA products and
-// 64 threads, 10.8 ms so (RZ then still on both halves).
+// 64 threads, 10.8 ms so.
 #ifndef SPZ_ADJ_THREADS
 #define SPZ_ADJ_THREADS 128
 #endif
@@ -473,7 +473,7 @@ int apply_hamiltonian(spz_state_t h, const spz_pauli_term* terms, size_t nterms,
     double c8[8];
     const int count = (int)std::min<size_t>(8, diag.size() - ch * 8);
     for (int b = 0; b < count; ++b) c8[b] = terms[diag[ch * 8 + b]].coeff;
-    for (int v = 0; v < 256; ++v) tab[ch * 256 + v] = signed_sum(c8, count, v);
+    for (int v = 0; v < (1 << count); ++v) tab[ch * 256 + v] = signed_sum(c8, count, v);
   }
   void* scratch;
   int rc = ensure_dev_scratch(h, tab.size() * sizeof(double), &scratch);

@@ -615,7 +615,7 @@ static int pauli_tiles(spz_state_t h, const spz_pauli_term* terms, size_t nterms
     double c[8];
     const int count = (int)std::min<size_t>(8, nd - ch * 8);
     for (int b = 0; b < count; ++b) c[b] = terms[diag[ch * 8 + b]].coeff;
-    for (int v = 0; v < 256; ++v) tab[ch * 256 + v] = signed_sum(c, count, v);
+    for (int v = 0; v < (1 << count); ++v) tab[ch * 256 + v] = signed_sum(c, count, v);
   }
   const int blocks = (int)std::min<uint64_t>(1ull << (n - k), (uint64_t)kNumSMs * 3);
   const size_t slots_per_pass = (size_t)(kPtMaxTerms + 1) * blocks;

@@ -42,15 +42,10 @@ __device__ __forceinline__ FxAmp fx_from_double(double re, double im) {
   return fx_from(dbits(re), dbits(im));
 }
 
-// parities of the index x = base | (tile offset e) under the op's masks
+// parities of the tile's base index under the op's masks
 __device__ __forceinline__ uint32_t fx_base_index(const TileGate& g, uint64_t base) {
   uint32_t idx = 0;
   for (int j = 0; j < g.pm; ++j) idx |= (uint32_t)(__popcll(base & g.pmask[j]) & 1) << j;
-  return idx;
-}
-__device__ __forceinline__ uint32_t fx_index(const TileGate& g, uint32_t bidx, uint32_t e) {
-  uint32_t idx = bidx;
-  for (int j = 0; j < g.pm; ++j) idx ^= (uint32_t)(__popc(e & g.pemask[j]) & 1) << j;
   return idx;
 }
 

@@ -38,50 +38,50 @@ struct TileMap {
 inline uint32_t parity32(uint32_t v) { return (uint32_t)__builtin_popcount(v) & 1u; }
 
 // The walk of op t under the map: items have the offset bits of t.e_mask fixed
-// (set where t.l_ones has them); `sel` are the offset masks whose parities come
-// in bits 16 and up of a word.
-inline void set_walk(TileGate* t, const TileMap& map, const std::vector<uint32_t>& sel) {
+// (set where t.l_ones has them); sel[0 .. nsel) are the offset masks whose parities
+// come in bits 16 and up of a word.  (On fixed arrays: an execute forms a walk per
+// gate, 0.3 us each with vectors, more than a small circuit's gate takes on the GPU.)
+inline void set_walk(TileGate* t, const TileMap& map, const uint32_t* sel, int nsel) {
   struct Fn {
     uint32_t f, xs, v;  // parity(p & f) = v ^ parity(x & xs)
   };
-  std::vector<Fn> fn;
-  std::vector<int> piv;
-  for (int q = 0; q < map.k; ++q) {
-    if (!((t->e_mask >> q) & 1)) continue;
+  Fn fn[kTileMaxK];
+  int piv[kTileMaxK], nf = 0;
+  uint32_t fixed = 0;
+  for (uint32_t left = t->e_mask & ((1u << map.k) - 1u); left; left &= left - 1) {
+    const int q = __builtin_ctz(left);
     Fn n{map.row[q], 1u << q, (t->l_ones >> q) & 1u};
-    for (size_t i = 0; i < fn.size(); ++i)
+    for (int i = 0; i < nf; ++i)
       if ((n.f >> piv[i]) & 1) n = Fn{n.f ^ fn[i].f, n.xs ^ fn[i].xs, n.v ^ fn[i].v};
     const int p = 31 - __builtin_clz(n.f);  // highest bit: the low slot bits stay with the low bits of m
-    for (Fn& o : fn)
-      if ((o.f >> p) & 1) o = Fn{o.f ^ n.f, o.xs ^ n.xs, o.v ^ n.v};
-    fn.push_back(n);
-    piv.push_back(p);
+    for (int i = 0; i < nf; ++i)
+      if ((fn[i].f >> p) & 1) fn[i] = Fn{fn[i].f ^ n.f, fn[i].xs ^ n.xs, fn[i].v ^ n.v};
+    fn[nf] = n;
+    piv[nf++] = p;
+    fixed |= 1u << p;
   }
-  uint32_t fixed = 0;
-  for (int p : piv) fixed |= 1u << p;
-  std::vector<uint32_t> g(sel.size(), 0);
-  for (size_t l = 0; l < sel.size(); ++l)
-    for (int q = 0; q < map.k; ++q)
-      if ((sel[l] >> q) & 1) g[l] ^= map.row[q];
+  uint32_t g[16] = {};  // sel as masks of the slot
+  for (int l = 0; l < nsel; ++l)
+    for (uint32_t left = sel[l]; left; left &= left - 1) g[l] ^= map.row[__builtin_ctz(left)];
   auto with_sel = [&](uint32_t p, uint32_t e) {  // e: offset bits that x adds beside the slot
-    for (size_t l = 0; l < sel.size(); ++l) p |= (parity32(p & 0xFFFFu & g[l]) ^ parity32(e & sel[l])) << (16 + l);
+    for (int l = 0; l < nsel; ++l) p |= (parity32(p & 0xFFFFu & g[l]) ^ parity32(e & sel[l])) << (16 + l);
     return p;
   };
   int m = 0;
   for (int b = 0; b < map.k; ++b) {
     if ((fixed >> b) & 1) continue;
     uint32_t p = 1u << b;
-    for (size_t j = 0; j < fn.size(); ++j)
+    for (int j = 0; j < nf; ++j)
       if ((fn[j].f >> b) & 1) p |= 1u << piv[j];
     t->wcol[m++] = with_sel(p, 0);
   }
   for (; m < 12; ++m) t->wcol[m] = 0;
   uint32_t k0 = 0;
-  for (size_t j = 0; j < fn.size(); ++j) k0 |= fn[j].v << piv[j];
+  for (int j = 0; j < nf; ++j) k0 |= fn[j].v << piv[j];
   t->wk0 = with_sel(k0, 0);
   for (int q = 0; q < kTileMaxK; ++q) {
     uint32_t p = 0;
-    for (size_t j = 0; j < fn.size(); ++j) p |= ((fn[j].xs >> q) & 1u) << piv[j];
+    for (int j = 0; j < nf; ++j) p |= ((fn[j].xs >> q) & 1u) << piv[j];
     t->wx[q] = q < map.k ? with_sel(p, 1u << q) : 0;
   }
   auto slot_of = [&](uint32_t bit) { return bit ? map.col[__builtin_ctz(bit)] : 0u; };
@@ -96,6 +96,7 @@ inline void map_pass(std::vector<TileGate>* ops, int k, bool keep_moves) {
   TileMap map(k);
   bool x_set = false;  // x may be other than 0
   std::vector<TileGate> out;
+  out.reserve(ops->size() + 1);
   for (TileGate& t : *ops) {
     const bool anywhere = t.g_ones == 0 && t.g_zeros == 0 && t.cond < 0;
     const uint32_t local = t.e_mask & ~t.tbit;  // of an X: its controls inside the tile
@@ -122,11 +123,8 @@ inline void map_pass(std::vector<TileGate>* ops, int k, bool keep_moves) {
       if (x_set) out.push_back(t);
       continue;
     }
-    std::vector<uint32_t> sel;
-    if (t.mode == TM_DIAG_LOCAL) sel.push_back(t.tbit);
-    else
-      for (int j = 0; j < t.pm; ++j) sel.push_back(t.pemask[j]);
-    set_walk(&t, map, sel);
+    if (t.mode == TM_DIAG_LOCAL) set_walk(&t, map, &t.tbit, 1);
+    else set_walk(&t, map, t.pemask, t.pm);
     out.push_back(t);
   }
   TileGate end{};  // item m: the slot of offset 2 m; tmask: what offset 2 m + 1 adds
